@@ -119,7 +119,10 @@ __device__ OrderSums order_sums(const LocalParams& p, int im, double x, double s
 		const double dy2 = a * (x * dy1 - s2 * y1) + b * dy0;
 		y0 = y1; y1 = y2; dy0 = dy1; dy1 = dy2;
 		if (E && fabs(y1) > LOC_BIG) {
-			if (E >= -LOC_FOLD) {
+			// fold when that leaves the value above 2^-LOC_FOLD: an exponent
+			// that stays is below -LOC_FOLD, so that the terms left out (E != 0)
+			// are below 2^(500 - LOC_FOLD)
+			if (E >= -LOC_FOLD - 500) {
 				y0 = ldexp(y0, E); y1 = ldexp(y1, E); dy0 = ldexp(dy0, E); dy1 = ldexp(dy1, E); E = 0;
 			} else {
 				y0 *= 0x1p-500; y1 *= 0x1p-500; dy0 *= 0x1p-500; dy1 *= 0x1p-500; E += 500;

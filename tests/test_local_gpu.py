@@ -169,6 +169,22 @@ def test_points_high_degree_against_long_double():
     assert relerr(ref, got) < TOL
 
 
+def test_points_with_seeds_far_below_the_double_range():
+    """lmax 2047 at sin(theta) = 0.5 and 0.7: orders whose seed sin^(m-1)
+    starts below 2^-600 and whose Legendre functions still grow to O(1) within
+    the degrees kept.  Bound: the recurrence's rounding (about lmax 2^-52 of the
+    largest value) and that of the phase m phi (lmax phi 2^-53), with a factor 4."""
+    import shtns_b200
+    from oracle.sht_ld import synth_points
+    lmax = 2047
+    sh = shtns_b200.sht(lmax)
+    q = rand_spec(lmax, lmax, 1, 78)
+    xs, phis = np.array([np.sqrt(0.75), -np.sqrt(0.51)]), np.array([0.3, 2.0])
+    ref = synth_points(q, lmax, xs, phis)
+    got = np.array([[sh.SH_to_point(q, x, ph) for ph in phis] for x in xs])
+    assert relerr(ref, got) < 4 * lmax * 2.0 ** -52
+
+
 def test_batched_points_equal_single_points():
     import torch
     import shtns_b200
