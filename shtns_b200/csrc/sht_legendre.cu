@@ -114,15 +114,20 @@ __global__ void ck_kernel(int nlat_2, int mres, int seg, const double* __restric
 // Column layout: field-component fc owns columns 16*(fc/4) + 2*(fc%4) + {0,1}
 // (even re, im) and the same +8 (odd re, im).
 //
-// CTA = (order im, 32 Ishioka rows k, 16 field-components): the degree window
-// [2k0-1, 2k0+66] of each input array is staged in shared memory with
-// coalesced loads, then every qq row segment is written contiguously.
-#define PT_K 32
-#define PT_F 16
-#define PT_W 69          // window length (68 needed), odd stride in 16-byte units
+// CTA = (order im, PT_K = pt_items / PF Ishioka rows k, PF field-components): the degree
+// window [2 k0 - 1, 2 k0 + 2 PT_K + 2] of each input array is staged in shared
+// memory with coalesced loads, then every qq row segment is written
+// contiguously.  PF is the power of two up to 16 that the call's
+// field-components fill best (launch_prep_synth): with 16 for every call, one
+// qst field at lmax 1023 kept 3 of 16 lanes and took 68 us instead of 35 (8
+// scalar fields at lmax 4095: 684 instead of 452).
+__host__ __device__ constexpr int pt_items(int PF) { return PF <= 2 ? 256 : 512; }     // (row, field-component) items of a CTA
 
+template <int PF>
 __global__ void __launch_bounds__(256, 6) prep_synth_kernel(PrepParams p)
 {
+	constexpr int PT_F = PF, PT_K = pt_items(PF) / PF;
+	constexpr int PT_W = 2 * PT_K + 5;       // window length, odd stride in 16-byte units
 	__shared__ double2 win[2][PT_F][PT_W];
 	__shared__ double cfs[2][PT_W];          // sin d/dtheta coupling (lo, hi) of the window's degrees
 	__shared__ double xk[3 * PT_K];          // basis change X of the CTA's k rows
@@ -141,60 +146,70 @@ __global__ void __launch_bounds__(256, 6) prep_synth_kernel(PrepParams p)
 	const int d0 = 2 * k0 - 1;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int voff = p.mt.voff[im];
+	const bool vec = p.comp_type[0] != 0 || p.ncomp > 1;
 	if (tid < PT_F) {
 		const int fc = fc0 + tid;
 		const int comp = fc / p.nf;
 		s_comp[tid] = (fc < nfc) ? comp : -1;
 		s_f[tid] = fc - comp * p.nf;
-	} else if (tid >= 32 && tid < 32 + PT_W) {
-		const int i = tid - 32, d = d0 + i;
-		cfs[0][i] = (d > 0 && d <= lrel_max + 1) ? p.stdt_lo[voff + d] : 0.0;
-		cfs[1][i] = (d >= 0 && d <= lrel_max + 1) ? p.stdt_hi[voff + d] : 0.0;
-	} else if (tid >= 128 && tid < 128 + 3 * PT_K) {
-		const int e = tid - 128;
-		xk[e] = (k0 + e / 3 <= kmax) ? p.xs[p.mt.xoff[im] + 3 * k0 + e] : 0.0;
 	}
-	// window of degrees d0 .. d0 + 68 of each (array, field-component): warp w
-	// stages pairs w, w + 8, w + 16, w + 24 (array = pair / 16), lanes along
-	// the degrees, two pairs at a time with all their loads issued before the
-	// first store
-	constexpr int NI = (PT_W + 31) / 32;
+	if (vec)
+		for (int i = tid; i < PT_W; i += 256) {
+			const int d = d0 + i;
+			cfs[0][i] = (d > 0 && d <= lrel_max + 1) ? p.stdt_lo[voff + d] : 0.0;
+			cfs[1][i] = (d >= 0 && d <= lrel_max + 1) ? p.stdt_hi[voff + d] : 0.0;
+		}
+	for (int e = tid; e < 3 * PT_K; e += 256) xk[e] = (k0 + e / 3 <= kmax) ? p.xs[p.mt.xoff[im] + 3 * k0 + e] : 0.0;
+	// window of the degrees of each (array, field-component) pair (array =
+	// pair / PF, the second one for vectors only), lanes along the degrees: WP
+	// warps share a pair or a warp takes PW of them, QB pairs and up to UB loads
+	// of each before the first store
+	constexpr int WP = (2 * PF >= 8) ? 1 : 8 / (2 * PF), PW = (2 * PF >= 8) ? 2 * PF / 8 : 1;
+	constexpr int NI = (PT_W + 32 * WP - 1) / (32 * WP);
+	constexpr int QB = (PW >= 2 && NI <= 3) ? 2 : 1, UB = (NI <= 5) ? NI : (NI + 1) / 2;
+	const int q0 = (WP == 1) ? warp : warp / WP, i0 = lane + 32 * (warp % WP);
 	#pragma unroll
-	for (int h = 0; h < 2; h++) {
-		double2 v[2][NI];
+	for (int h = 0; h < PW; h += QB) {
+		const double2* base[QB];
 		#pragma unroll
-		for (int qi = 0; qi < 2; qi++) {
-			const int q = warp + 8 * (2 * h + qi), a = q / PT_F, fl = q % PT_F;
-			const int fc = fc0 + fl;
-			const double2* base = nullptr;
-			if (fc < nfc) {
+		for (int qi = 0; qi < QB; qi++) {
+			const int q = q0 + 8 * (h + qi), a = q / PT_F, fc = fc0 + q % PT_F;
+			base[qi] = nullptr;
+			if (fc < nfc && (a == 0 || vec)) {
 				const int comp = fc / p.nf, f = fc - comp * p.nf;
-				base = (p.comp_type[comp] == 0) ? (a == 0 ? p.Q : nullptr) : (a == 0 ? p.S : p.T);
-				if (base) base += off + (long)f * p.spec_dist;
-			}
-			#pragma unroll
-			for (int u = 0; u < NI; u++) {
-				const int d = d0 + lane + 32 * u;
-				v[qi][u] = (base && lane + 32 * u < PT_W && d >= 0 && d <= lrel_max) ? base[d] : make_double2(0.0, 0.0);
+				const double2* x = (p.comp_type[comp] == 0) ? (a == 0 ? p.Q : nullptr) : (a == 0 ? p.S : p.T);
+				if (x) base[qi] = x + off + (long)f * p.spec_dist + d0;
 			}
 		}
 		#pragma unroll
-		for (int qi = 0; qi < 2; qi++) {
-			const int q = warp + 8 * (2 * h + qi), a = q / PT_F, fl = q % PT_F;
+		for (int u0 = 0; u0 < NI; u0 += UB) {
+			double2 v[QB][UB];
 			#pragma unroll
-			for (int u = 0; u < NI; u++) {
-				const int i = lane + 32 * u;
-				if (i < PT_W) {
-					double2 x = v[qi][u];
-					if (m0) x.y = 0.0;
-					win[a][fl][i] = x;
+			for (int qi = 0; qi < QB; qi++)
+				#pragma unroll
+				for (int u = 0; u < UB; u++) {
+					const int i = i0 + 32 * WP * (u0 + u), d = d0 + i;
+					v[qi][u] = make_double2(0.0, 0.0);
+					if (u0 + u < NI && base[qi] && i < PT_W && d >= 0 && d <= lrel_max) {
+						const double2 x = base[qi][i];
+						v[qi][u] = make_double2(x.x, m0 ? 0.0 : x.y);
+					}
+				}
+			#pragma unroll
+			for (int qi = 0; qi < QB; qi++) {
+				const int q = q0 + 8 * (h + qi), a = q / PT_F, fl = q % PT_F;
+				if (a != 0 && !vec) continue;
+				#pragma unroll
+				for (int u = 0; u < UB; u++) {
+					const int i = i0 + 32 * WP * (u0 + u);
+					if (u0 + u < NI && i < PT_W) win[a][fl][i] = v[qi][u];
 				}
 			}
 		}
 	}
 	__syncthreads();
 	const double em = (p.msign < 0) ? -(double) m : (double) m;   // signed m (negative orders of the _ml transforms)
-	for (int e = tid; e < PT_K * PT_F; e += blockDim.x) {
+	for (int e = tid; e < PT_K * PT_F; e += 256) {
 		const int kl = e / PT_F, fl = e - kl * PT_F;
 		const int k = k0 + kl, fc = fc0 + fl;
 		if (k >= kmax || fc >= nfc) continue;
@@ -239,16 +254,22 @@ __global__ void __launch_bounds__(256, 6) prep_synth_kernel(PrepParams p)
 // with MX = 2 cos + sin d/dtheta (SH_2scal_to_vect, sht_private.h:296-337).
 // Degrees above llim and orders above mlim are written as zero (SHT_VAR_LTR).
 //
-// CTA = (order im, 64 degrees, 16 fields, output group): the k rows covering
+// CTA = (order im, PE_J degrees, PF fields, output group): the k rows covering
 // the degree tile plus one row of halo on each side are staged in shared
-// memory for the (one or two) field-components of the group.
-#define PE_J 64
-#define PE_F 16
-#define PE_R 36          // staged k rows: j0/2-2 .. j0/2+33
-#define PE_S (2 * PE_F + 2)   // row stride in double2: 32 mod 128 bytes, so the 4 rows read by 8 lanes use distinct banks
+// memory for the (one or two) field-components of the group.  PF (1, 4, 8 or
+// 16) is what the call's fields fill best; with 16 for every call, one qst
+// field at lmax 1023 took 118 us instead of 35 (8 scalar fields at lmax 4095:
+// 831 instead of 523).
+template <int PF>
+struct PostTile {
+	static constexpr int J = (PF == 1) ? 512 : (PF == 4) ? 128 : 1024 / PF;   // degrees
+	static constexpr int R = J / 2 + 4;                     // staged k rows: j0/2-2 .. j0/2+J/2+1
+	static constexpr int S = (PF == 1) ? 2 : 2 * PF + 2;    // row stride in double2: 32 mod 128 bytes, so the 4 rows read by 8 lanes use distinct banks
+};
 
 // E[row][2 fl + 0] = even pair (re, im), [2 fl + 1] = odd pair, row = k - kb;
 // Xs[3 row + c] = basis-change coefficients of k
+template <int PE_S>
 __device__ __forceinline__ double2 ish_inv_s(const double2 (*E)[PE_S], const double* Xs, int kb, int fl, int j)
 {
 	if (j < 0) return make_double2(0.0, 0.0);
@@ -270,8 +291,10 @@ __device__ __forceinline__ double2 ish_inv_s(const double2 (*E)[PE_S], const dou
 	return make_double2(x2 * o.x, x2 * o.y);
 }
 
+template <int PF>
 __global__ void __launch_bounds__(256) post_analys_kernel(PrepParams p)
 {
+	constexpr int PE_F = PF, PE_J = PostTile<PF>::J, PE_R = PostTile<PF>::R, PE_S = PostTile<PF>::S;
 	constexpr int NE = PE_R * PE_F * 2, NU = (NE + 255) / 256;
 	__shared__ double2 sv[PE_R][PE_S];     // first component of the group (Q, or V)
 	__shared__ double2 sw[PE_R][PE_S];     // second component (W) for the vector group
@@ -800,12 +823,34 @@ void launch_checkpoints(shtns_cfg s, cudaStream_t st)
 	cudaFree(d_nseg);
 }
 
+// Fields (or field-components) per CTA of the prologue and epilogue kernels: 1
+// or 2 for so many, else the largest of 16, 8 and 4 that leaves the fewest
+// idle (fewer than 4 split the 64-byte groups of four field-components)
+static int tile_fields(int n)
+{
+	if (n <= 2) return n;
+	int best = 16;
+	for (int f = 8; f >= 4; f /= 2)
+		if ((n + f - 1) / f * f < (n + best - 1) / best * best) best = f;
+	return best;
+}
+
 void launch_prep_synth(const PrepParams& p, cudaStream_t st)
 {
 	const int nfc = p.nf * p.ncomp;
 	const int kmax0 = (p.llim + 1) / 2 + 1;
-	dim3 grid((kmax0 + PT_K - 1) / PT_K, (nfc + PT_F - 1) / PT_F, p.mlim + 1 - p.im0);
-	prep_synth_kernel<<<grid, 256, 0, st>>>(p);
+	auto go = [&](auto kern, int PF) {
+		const int K = pt_items(PF) / PF;
+		dim3 grid((kmax0 + K - 1) / K, (nfc + PF - 1) / PF, p.mlim + 1 - p.im0);
+		kern<<<grid, 256, 0, st>>>(p);
+	};
+	switch (tile_fields(nfc)) {
+		case 1: go(prep_synth_kernel<1>, 1); break;
+		case 2: go(prep_synth_kernel<2>, 2); break;
+		case 4: go(prep_synth_kernel<4>, 4); break;
+		case 8: go(prep_synth_kernel<8>, 8); break;
+		default: go(prep_synth_kernel<16>, 16); break;
+	}
 	shtb_count_launch();
 }
 
@@ -882,9 +927,16 @@ void launch_leg_analys(const LegParams& p, int kmax_all, cudaStream_t st)
 void launch_post_analys_m(const PrepParams& p, int mmax, cudaStream_t st)
 {
 	const int ngroups = (p.comp_type[0] == 0) ? 1 + (p.ncomp > 1 ? 1 : 0) : 1;
-	const int nft = (p.nf + PE_F - 1) / PE_F;
-	dim3 grid((p.lmax + 1 + PE_J - 1) / PE_J, nft * ngroups, mmax + 1 - p.im0);
-	post_analys_kernel<<<grid, 256, 0, st>>>(p);
+	auto go = [&](auto kern, int PF, int J) {
+		dim3 grid((p.lmax + J) / J, (p.nf + PF - 1) / PF * ngroups, mmax + 1 - p.im0);
+		kern<<<grid, 256, 0, st>>>(p);
+	};
+	switch (tile_fields(p.nf)) {
+		case 1: go(post_analys_kernel<1>, 1, PostTile<1>::J); break;
+		case 2: case 4: go(post_analys_kernel<4>, 4, PostTile<4>::J); break;
+		case 8: go(post_analys_kernel<8>, 8, PostTile<8>::J); break;
+		default: go(post_analys_kernel<16>, 16, PostTile<16>::J); break;
+	}
 	shtb_count_launch();
 }
 
