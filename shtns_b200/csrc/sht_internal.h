@@ -260,6 +260,8 @@ void launch_ptab_analys(shtns_cfg s, const LegParams& p, cudaStream_t st);
 void free_ptab(shtns_cfg s);
 bool launch_ftab_synth(shtns_cfg s, const LegParams& p, cudaStream_t st);
 void free_ftab(shtns_cfg s);
+void launch_leg_synth_narrow(const LegParams& p, cudaStream_t st);
+void launch_leg_analys_narrow(const LegParams& p, int kmax_all, cudaStream_t st);
 bool leg_simt_selected(const LegParams& p, bool synth);
 void launch_leg_synth_simt(const LegParams& p, cudaStream_t st);
 void launch_leg_analys_simt(const LegParams& p, int kmax_all, cudaStream_t st);

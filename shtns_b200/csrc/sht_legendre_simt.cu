@@ -489,14 +489,23 @@ void analys_seg(const LegParams& p, dim3 grid, int nt, cudaStream_t st)
 } // namespace
 
 // Calls with 1..4 field-components take the SIMT kernels when the tile option
-// asks for them (8) or, automatically (0), up to 4 components in the synthesis
-// and 3 in the analysis (measured on B200 at lmax 511, 1023 and 4095: with 4
-// components the tensor-core analysis tiles are faster below lmax 4095).
+// asks for them (8) or, automatically (0), where they beat the 128 x 16 tensor-core
+// tiles.  Measured on B200 (us, SIMT / tiles, lmax 127, 340, 511, 1023, 2047):
+//   analysis  1 component   9.8/14.5  27/37  58/55  270/276  1585/1852
+//             2             19.7/14.3  44/37  86/54  345/278
+//             3             20.2/14.8  48/37  86/54  424/283  2790/1879
+//   synthesis 2             18.8/17.8  30/31  47/53  181/281
+//             3             22.9/17.4  35/31  65/53  258/285  1692/1945
+//             4             39/31 (340)  77/53  329/287  2225/1952
+// so: the analysis of one component; the synthesis of one and two, and of
+// three where the grid has more than 1024 rows.
 bool leg_simt_selected(const LegParams& p, bool synth)
 {
 	if (p.nfc < 1 || p.nfc > 4) return false;
 	if (p.tile_wm == 8) return true;
-	return p.tile_wm == 0 && p.nfc <= (synth ? 4 : 3);
+	if (p.tile_wm != 0) return false;
+	if (synth) return p.nfc <= 2 || (p.nfc == 3 && p.nlat_2 > 512);
+	return p.nfc == 1;
 }
 
 void launch_leg_synth_simt(const LegParams& p, cudaStream_t st)
