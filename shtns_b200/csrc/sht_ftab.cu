@@ -409,14 +409,19 @@ bool ft_err_flag(shtns_cfg s, cudaStream_t st)
 
 } // namespace
 
-// The table form runs the 64 x 64 tile shape (the automatic choice above 32
-// GEMM columns, or option 5 = 2) on the plain Fourier buffer; it returns false
+// The table form runs the 64 x 64 tile shape on the plain Fourier buffer:
+// automatically with more than 128 GEMM columns (32 field-components), or with
+// option 5 = 2 or option 10 = 2 above 32.  With one or two column tiles a table
+// block is read from HBM for little work: measured (us, table / on the fly)
+// lmax 511, 13 fields 124/119, 32 fields 227/230, 64 fields 429/447; lmax 1023,
+// 13 fields 817/776, 32 fields 1551/1548; lmax 359, 13 fields 73/68, 40 fields
+// 172/175; lmax 255, 64 field-components 55/59.  It returns false
 // (the caller launches the on-the-fly kernels) when it does not apply or the
 // table does not fit the automatic budget.
 bool launch_ftab_synth(shtns_cfg s, const LegParams& p, cudaStream_t st)
 {
 	if (s->ftab_mode == 1 || p.rb.n) return false;
-	if (!(p.tile_wm == 2 || (p.tile_wm == 0 && p.ncol > 32))) return false;
+	if (!(p.tile_wm == 2 || (p.tile_wm == 0 && p.ncol > (s->ftab_mode == 2 ? 32 : 128)))) return false;
 	if (leg_simt_selected(p, true)) return false;
 	shtns_cfg o = s->is_clone ? s->base : s;
 	if (!ftab_ensure(o, s->ftab_mode == 2, st)) return false;
