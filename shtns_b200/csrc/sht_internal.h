@@ -170,7 +170,8 @@ struct LegParams {
 	int nlat, nlat_2, llim, mlim, mres, vec_extra;
 	int im0;                             // first order of the launch (orders im0..mlim; 0 for whole transforms)
 	int ncol, nfc;
-	int ckseg;                           // checkpoint spacing in k (8, 16 or 32)
+	int ckseg;                           // checkpoint spacing in k (8, 16 or 32) that the kernel uses
+	int ckrow;                           // checkpoints between two of its segments (nlat_2, or more where it skips some of the table's)
 	int tile_wm;                         // Legendre tile: warps along the rows (1, 2, 4; 0 automatic)
 	int south_first, robert;
 	double mpos_inv;                     // analysis factor for m>0 (1/mpos_renorm)
@@ -262,6 +263,7 @@ bool launch_ftab_synth(shtns_cfg s, const LegParams& p, cudaStream_t st);
 void free_ftab(shtns_cfg s);
 void launch_leg_synth_narrow(const LegParams& p, cudaStream_t st);
 void launch_leg_analys_narrow(const LegParams& p, int kmax_all, cudaStream_t st);
+LegParams leg_spaced(const LegParams& p, int want);
 bool leg_simt_selected(const LegParams& p, bool synth);
 void launch_leg_synth_simt(const LegParams& p, cudaStream_t st);
 void launch_leg_analys_simt(const LegParams& p, int kmax_all, cudaStream_t st);

@@ -528,9 +528,27 @@ static int tile_wm(const LegParams& p, bool synth)
 	return (synth || p.nlat_2 > 256) ? 5 : 4;
 }
 
-void launch_leg_synth(const LegParams& p, cudaStream_t st)
+// Segments of at least `want` steps from a table of denser checkpoints: the
+// recurrence reaches the values of the checkpoints it passes over exactly.
+LegParams leg_spaced(const LegParams& p, int want)
 {
-	if (leg_simt_selected(p, true)) { launch_leg_synth_simt(p, st); shtb_count_launch(); return; }
+	LegParams q = p;
+	while (q.ckseg < want) { q.ckseg *= 2; q.ckrow *= 2; }
+	return q;
+}
+
+// 64 x 64 tiles: 8 steps per segment, so that every thread generates one of the
+// shortest chains (lmax 1023, 32 fields, synthesis / analysis: 8: 1553/1655 us, 16:
+// 1671/1707).  128 rows: 16 steps keep every thread busy too and read half of
+// the checkpoints (lmax 511, 8 fields: 8: 83/91 us, 16: 78/84; lmax 1023, 8 fields:
+// 8: 491/454, 16: 468/451, 32: 541/491; lmax 2047: 3.48/3.25 ms, 3.35/3.21,
+// 3.81/3.42).
+static int tile_spacing(int wm) { return wm == 2 ? 8 : 16; }
+
+void launch_leg_synth(const LegParams& p0, cudaStream_t st)
+{
+	if (leg_simt_selected(p0, true)) { launch_leg_synth_simt(p0, st); shtb_count_launch(); return; }
+	const LegParams p = leg_spaced(p0, tile_spacing(tile_wm(p0, true)));
 	switch (tile_wm(p, true)) {
 		case 1: launch_leg_synth_wm<1>(p, st); break;
 		case 4: launch_leg_synth_wm<4>(p, st); break;
@@ -540,9 +558,10 @@ void launch_leg_synth(const LegParams& p, cudaStream_t st)
 	shtb_count_launch();
 }
 
-void launch_leg_analys(const LegParams& p, int kmax_all, cudaStream_t st)
+void launch_leg_analys(const LegParams& p0, int kmax_all, cudaStream_t st)
 {
-	if (leg_simt_selected(p, false)) { launch_leg_analys_simt(p, kmax_all, st); shtb_count_launch(); return; }
+	if (leg_simt_selected(p0, false)) { launch_leg_analys_simt(p0, kmax_all, st); shtb_count_launch(); return; }
+	const LegParams p = leg_spaced(p0, tile_spacing(tile_wm(p0, false)));
 	switch (tile_wm(p, false)) {
 		case 1: launch_leg_analys_wm<1>(p, kmax_all, st); break;
 		case 4: launch_leg_analys_wm<4>(p, kmax_all, st); break;

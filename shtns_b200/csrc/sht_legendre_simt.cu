@@ -120,8 +120,8 @@ __global__ void __launch_bounds__(128) leg_synth_simt_kernel(LegParams p)
 				const int sg = (k0 + s0) / SEG;
 				double ya0 = na.x, ya1 = na.y, yc0 = nc.x, yc1 = nc.y;
 				const bool more = k0 + s0 + SEG < nk;     // checkpoint of the next segment, loaded ahead
-				na = (la && more) ? __ldg(ckm + (long)(sg + 1) * p.nlat_2 + ta) : z;
-				nc = (lc && more) ? __ldg(ckm + (long)(sg + 1) * p.nlat_2 + tc) : z;
+				na = (la && more) ? __ldg(ckm + (long)(sg + 1) * p.ckrow + ta) : z;
+				nc = (lc && more) ? __ldg(ckm + (long)(sg + 1) * p.ckrow + tc) : z;
 				const double* c = cs + s0 * W;
 				simt_acc<NFC>(aa, c, ya0);
 				simt_acc<NFC>(ac, c, yc0);
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(SA_NT) leg_analys_simt_kernel(LegParams p)
 		#pragma unroll
 		for (int u = 0; u < SPT; u++) {
 			const int ks = kb0 + (gs + u * ngs) * SEG;
-			ckn[u] = (t < p.nlat_2 && t >= tmm && ks < nk) ? __ldg(ckm + (long)(ks / SEG) * p.nlat_2 + t)
+			ckn[u] = (t < p.nlat_2 && t >= tmm && ks < nk) ? __ldg(ckm + (long)(ks / SEG) * p.ckrow + t)
 			                                              : make_double2(0.0, 0.0);
 		}
 		#pragma unroll
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(SR_NT) leg_analys_reg_kernel(LegParams p)
 		#pragma unroll
 		for (int b = 0; b < NSB; b++) {
 			const int ks = (NSB > 1) ? kb0 + b * SEG : s0;
-			nck[b] = (ks < nk) ? __ldg(ckm + (long)(ks / SEG) * p.nlat_2 + t) : make_double2(0.0, 0.0);
+			nck[b] = (ks < nk) ? __ldg(ckm + (long)(ks / SEG) * p.ckrow + t) : make_double2(0.0, 0.0);
 		}
 		nw = p.adjoint ? 0.0 : __ldg(p.w + t);
 		nx = __ldg(p.x + t);
@@ -472,7 +472,6 @@ template <int SEG, bool RB>
 void analys_seg_rb(const LegParams& p, dim3 grid, int nt, cudaStream_t st)
 {
 	switch (p.nfc) {
-		case 1: leg_analys_simt_kernel<SEG, 1, RB><<<grid, nt, 0, st>>>(p); break;
 		case 2: leg_analys_simt_kernel<SEG, 2, RB><<<grid, nt, 0, st>>>(p); break;
 		case 3: leg_analys_simt_kernel<SEG, 3, RB><<<grid, nt, 0, st>>>(p); break;
 		default: leg_analys_simt_kernel<SEG, 4, RB><<<grid, nt, 0, st>>>(p); break;
@@ -508,8 +507,12 @@ bool leg_simt_selected(const LegParams& p, bool synth)
 	return p.nfc == 1;
 }
 
-void launch_leg_synth_simt(const LegParams& p, cudaStream_t st)
+void launch_leg_synth_simt(const LegParams& p0, cudaStream_t st)
 {
+	// the chains of a segment stay in registers: the longest segments read the
+	// fewest checkpoints (lmax 127 to 1023, one component, 8 -> 32: 16.1 -> 14.7,
+	// 37 -> 33, 118 -> 112 us)
+	const LegParams p = leg_spaced(p0, 32);
 	const int half = (p.nlat_2 + 1) / 2;
 	const int nt = std::min(128, std::max(32, (half + 31) / 32 * 32));
 	dim3 grid((p.nlat_2 + 2 * nt - 1) / (2 * nt), p.mlim + 1 - p.im0);
@@ -528,9 +531,11 @@ void analys_reg_seg(const LegParams& p, int kmax_all, cudaStream_t st)
 	else leg_analys_reg_kernel<SEG, false><<<grid, SR_NT, 0, st>>>(p);
 }
 
-void launch_leg_analys_simt(const LegParams& p, int kmax_all, cudaStream_t st)
+void launch_leg_analys_simt(const LegParams& p0, int kmax_all, cudaStream_t st)
 {
-	if (p.nfc == 1 && (p.ckseg >= 16 || p.nlat_2 <= 512)) {
+	if (p0.nfc == 1) {
+		// as the synthesis (lmax 511, 767, 1023: 58 -> 54, 146 -> 131, 284 -> 262 us)
+		const LegParams p = leg_spaced(p0, 32);
 		switch (p.ckseg) {
 			case 8: analys_reg_seg<8>(p, kmax_all, st); break;
 			case 16: analys_reg_seg<16>(p, kmax_all, st); break;
@@ -538,6 +543,7 @@ void launch_leg_analys_simt(const LegParams& p, int kmax_all, cudaStream_t st)
 		}
 		return;
 	}
+	const LegParams& p = p0;
 	// block of 2 nt k: the smallest of 32, 64, 128 threads that covers kmax_all
 	int nt = 32;
 	while (nt < SA_NT && 2 * nt < kmax_all) nt *= 2;

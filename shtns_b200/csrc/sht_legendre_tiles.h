@@ -106,7 +106,7 @@ __device__ __forceinline__ void leg_synth_tile(const LegParams& p, int im, int t
 			for (int u = 0; u < SPT; u++) {
 				const int sg = gj + u * GPR;
 				const int ks = k0 + sg * SEG;
-				ckn[u] = (sg < NSEGC && gen && ks < nk) ? ldg_stream(ckm + (long)(ks / SEG) * p.nlat_2 + tg)
+				ckn[u] = (sg < NSEGC && gen && ks < nk) ? ldg_stream(ckm + (long)(ks / SEG) * p.ckrow + tg)
 				                                       : make_double2(0.0, 0.0);
 			}
 		};
@@ -288,7 +288,7 @@ __device__ __forceinline__ void leg_analys_tile(const LegParams& p, int im, int 
 		#pragma unroll
 		for (int u = 0; u < SPT; u++) {
 			const int sg = gsg + u * GPT, gks = k0 + sg * SEG;
-			ckn[u] = (sg < NSG && t < p.nlat_2 && gks < nk) ? ldg_stream(ckm + (long)(gks / SEG) * p.nlat_2 + t)
+			ckn[u] = (sg < NSG && t < p.nlat_2 && gks < nk) ? ldg_stream(ckm + (long)(gks / SEG) * p.ckrow + t)
 			                                               : make_double2(0.0, 0.0);
 		}
 	};

@@ -404,7 +404,7 @@ leg_synth_split_kernel(LegParams p, const uint4* __restrict__ bsl, const int* __
 			double y0 = 0.0, y1 = 0.0;
 			if (rsc != 0.0 && ks < nk) {
 				const int kc = (ks / SEG) * SEG;
-				const double2 y = __ldg(ckm + (long)(kc / SEG) * p.nlat_2);
+				const double2 y = __ldg(ckm + (long)(kc / SEG) * p.ckrow);
 				y0 = y.x * rsc; y1 = y.y * rsc;     // scaling by 2^-e commutes with the recurrence
 				// advance to (Y_ks, Y_ks+1); Y_ks+1 may lie past the order's last
 				// step (coefficient rows are padded to whole 32-step segments)
