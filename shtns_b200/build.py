@@ -12,7 +12,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libshtns_b200.so")
 OBJDIR = os.path.join(HERE, "_build")
 
-SOURCES = ["sht_plan.cu", "sht_gauss.cu", "sht_api.cu", "sht_legendre.cu", "sht_legendre_simt.cu", "sht_legendre_narrow.cu", "sht_fft.cu", "sht_noalloc.cu", "sht_split.cu", "sht_ptab.cu", "sht_ftab.cu", "sht_local.cu", "sht_rotation.cu"]
+SOURCES = ["sht_plan.cu", "sht_gauss.cu", "sht_api.cu", "sht_legendre.cu", "sht_legendre_simt.cu", "sht_legendre_narrow.cu", "sht_fft.cu", "sht_fft_gen.cu", "sht_noalloc.cu", "sht_split.cu", "sht_ptab.cu", "sht_ftab.cu", "sht_local.cu", "sht_rotation.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2"]
 
@@ -33,7 +33,7 @@ def _stale(target, deps):
 
 def build(verbose=False, ptxas_info=False):
     os.makedirs(OBJDIR, exist_ok=True)
-    headers = [os.path.join(CSRC, h) for h in ("sht_internal.h", "sht_legendre_tiles.h", "sht_ptx.h")] + [
+    headers = [os.path.join(CSRC, h) for h in ("sht_internal.h", "sht_legendre_tiles.h", "sht_dft.h", "sht_fft_tma.h", "sht_fft_grid.h", "sht_ptx.h")] + [
         os.path.join(HERE, "..", "include", h) for h in ("shtns.h", "shtns_cuda.h", "shtns_b200.h")]
     objs = []
     for src in SOURCES:

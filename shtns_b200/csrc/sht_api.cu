@@ -100,27 +100,18 @@ FftParams fft_params(shtns_cfg s, const Job& j, int nrows)
 	FftParams p;
 	memset(&p, 0, sizeof(p));
 	p.N = s->nphi; p.nlat = s->nlat; p.mlim = j.mlim;
-	p.nradix = (int) s->fft_radix.size();
-	p.rcode = 0;
-	int rmin = 8;
-	for (int i = 0; i < p.nradix; i++) {
-		p.rcode |= (unsigned long long) s->fft_radix[i] << (4 * i);
-		rmin = std::min(rmin, s->fft_radix[i]);
-	}
-	(void) rmin;
-	// latitude pairs per CTA: the largest of 4, 2, 1 whose two shared-memory
-	// buffers fit in about 110 KB (two CTAs per SM); SHTNS_B200_FFT_PAIRS
-	// overrides (tuning knob, clamped to what fits in 227 KB).
+	p.gen = &s->fft_gen; p.gen_small = &s->fft_gen_small;
+	// latitude pairs per CTA of the fused kernels: the largest of 4, 2, 1
+	// whose two shared-memory buffers fit in about 110 KB (two CTAs per SM);
+	// SHTNS_B200_FFT_PAIRS overrides (tuning knob, clamped to what fits in 227 KB).
 	int S = 4;
 	while (S > 1 && fft_smem_bytes(s->nphi, S) > 112 * 1024) S /= 2;
 	int want = s->fft_pairs;
 	if (const char* e = getenv("SHTNS_B200_FFT_PAIRS")) want = atoi(e);
 	if (want == 1 || want == 2 || want == 4 || want == 8) {
-		// fused chains keep one buffer, the generic kernels two
-		const bool fused = fft_fused_available(s->nphi) && s->fft_generic != 1;
 		S = want;
-		while (S > 1 && fft_smem_bytes(s->nphi, S) / (fused ? 2 : 1) > 227 * 1024) S /= 2;
-		if (!fused && S > 4) S = 4;
+		while (S > 1 && fft_smem_bytes(s->nphi, S) / 2 > 227 * 1024) S /= 2;
+		p.pairs = want;
 	}
 	while (S > 1 && 2 * S > nrows) S /= 2;
 	p.S = S;
@@ -128,11 +119,11 @@ FftParams fft_params(shtns_cfg s, const Job& j, int nrows)
 	p.fstride = (long)(s->mmax + 1) * s->nlat;
 	p.nf = j.nf; p.spat_dist = s->spat_dist;
 	p.phi_contiguous = s->phi_contiguous;
-	// generic kernels need two buffers
-	p.generic = (s->fft_generic == 1) ? (fft_smem_bytes(s->nphi, 1) <= 227 * 1024 ? 1 : 0) : s->fft_generic;
+	p.generic = (s->fft_generic == 1 && !s->fft_gen.np) ? 0 : s->fft_generic;     // 12288 has a fused chain only
 	p.extra_tx = s->fft_extra_tx;
 	p.tw1 = s->d_tw4;
-	p.tw2 = s->d_tw4 ? s->d_tw4 + 96 : nullptr;
+	int f1 = 0, f2 = 0;
+	p.tw2 = (s->d_tw4 && fft_fourstep_factors(s->nphi, f1, f2)) ? s->d_tw4 + f1 : nullptr;
 	p.scratch = nullptr;
 	return p;
 }

@@ -7,8 +7,8 @@
 // Hermitian symmetry.  A tile is one field-component and 2*S consecutive
 // latitudes; its S complex sequences are transformed in shared memory by a
 // self-sorting Stockham chain.  Three kernel families:
-//   * generic kernels: one tile per CTA, mixed radices (8, 4, 2, 3, 5, 7)
-//     chosen at run time, two shared-memory buffers (any supported nphi);
+//   * generic kernels (sht_fft_gen.cu): one tile per CTA, radices 2 .. 16
+//     chosen at run time (any supported nphi);
 //   * fused kernels (fft3_*): nphi = 3 * 2^k with a compile-time radix chain
 //     in one padded in-place buffer, one tile per CTA;
 //   * prefetching kernels (fft4_*, the default up to nphi 3072): persistent
@@ -21,329 +21,20 @@
 // The spatial arrays are theta-contiguous (v[j*nlat + theta]) or
 // phi-contiguous (v[theta*nphi + j]).
 #include "sht_internal.h"
+#include "sht_dft.h"
+#include "sht_fft_tma.h"
+#include "sht_fft_grid.h"
 
-#include <cuda.h>
-#include <cudaTypedefs.h>
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 #include <cstdint>
 
 namespace {
 
-__device__ __forceinline__ double2 cmul(double2 a, double2 b)
-{
-	return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
-}
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-// multiply by sign*i
-__device__ __forceinline__ double2 mul_si(double2 a, int sign) { return sign > 0 ? make_double2(-a.y, a.x) : make_double2(a.y, -a.x); }
-
-template <int R> struct Dft;
-
-template <> struct Dft<2> {
-	static __device__ __forceinline__ void run(double2* u, int) {
-		double2 a = u[0], b = u[1];
-		u[0] = cadd(a, b); u[1] = csub(a, b);
-	}
-};
-template <> struct Dft<4> {
-	static __device__ __forceinline__ void run(double2* u, int s) {
-		double2 t0 = cadd(u[0], u[2]), t1 = csub(u[0], u[2]);
-		double2 t2 = cadd(u[1], u[3]), t3 = mul_si(csub(u[1], u[3]), s);
-		u[0] = cadd(t0, t2); u[2] = csub(t0, t2);
-		u[1] = cadd(t1, t3); u[3] = csub(t1, t3);
-	}
-};
-template <> struct Dft<8> {
-	static __device__ __forceinline__ void run(double2* u, int s) {
-		const double h = 0.70710678118654752440084436210485;
-		// radix-2 split into even / odd halves, each a 4-point DFT
-		double2 e[4] = {u[0], u[2], u[4], u[6]};
-		double2 o[4] = {u[1], u[3], u[5], u[7]};
-		Dft<4>::run(e, s);
-		Dft<4>::run(o, s);
-		// twiddles w8^q = exp(s*i*pi*q/4)
-		double2 o1 = make_double2(h * (o[1].x - s * o[1].y), h * (o[1].y + s * o[1].x));
-		double2 o2 = mul_si(o[2], s);
-		double2 o3 = make_double2(h * (-o[3].x - s * o[3].y), h * (-o[3].y + s * o[3].x));
-		u[0] = cadd(e[0], o[0]); u[4] = csub(e[0], o[0]);
-		u[1] = cadd(e[1], o1);   u[5] = csub(e[1], o1);
-		u[2] = cadd(e[2], o2);   u[6] = csub(e[2], o2);
-		u[3] = cadd(e[3], o3);   u[7] = csub(e[3], o3);
-	}
-};
-template <> struct Dft<3> {
-	static __device__ __forceinline__ void run(double2* u, int s) {
-		const double c1 = -0.5, s1 = s * 0.86602540378443864676372317075294;
-		double2 t = cadd(u[1], u[2]), d = csub(u[1], u[2]);
-		double2 mm = make_double2(fma(c1, t.x, u[0].x), fma(c1, t.y, u[0].y));
-		u[0] = cadd(u[0], t);
-		u[1] = make_double2(mm.x - s1 * d.y, mm.y + s1 * d.x);
-		u[2] = make_double2(mm.x + s1 * d.y, mm.y - s1 * d.x);
-	}
-};
-template <> struct Dft<5> {
-	static __device__ __forceinline__ void run(double2* u, int s) {
-		const double c1 = 0.30901699437494742410229341718282;   // cos(2pi/5)
-		const double c2 = -0.80901699437494742410229341718282;  // cos(4pi/5)
-		const double s1 = s * 0.95105651629515357211643933337938;  // sin(2pi/5)
-		const double s2 = s * 0.58778525229247312916870595463907;  // sin(4pi/5)
-		double2 a1 = cadd(u[1], u[4]), b1 = csub(u[1], u[4]);
-		double2 a2 = cadd(u[2], u[3]), b2 = csub(u[2], u[3]);
-		double2 x0 = u[0];
-		u[0] = cadd(x0, cadd(a1, a2));
-		double2 r1 = make_double2(x0.x + c1 * a1.x + c2 * a2.x, x0.y + c1 * a1.y + c2 * a2.y);
-		double2 r2 = make_double2(x0.x + c2 * a1.x + c1 * a2.x, x0.y + c2 * a1.y + c1 * a2.y);
-		// i*(s1 b1 + s2 b2) and i*(s2 b1 - s1 b2)
-		double2 i1 = make_double2(-(s1 * b1.y + s2 * b2.y), s1 * b1.x + s2 * b2.x);
-		double2 i2 = make_double2(-(s2 * b1.y - s1 * b2.y), s2 * b1.x - s1 * b2.x);
-		u[1] = cadd(r1, i1); u[4] = csub(r1, i1);
-		u[2] = cadd(r2, i2); u[3] = csub(r2, i2);
-	}
-};
-// 7-point DFT as a direct sum with the roots of unity as literals
-// (cos, sin of 2 pi k / 7, symmetric pairs folded).
-template <> struct Dft<7> {
-	static __device__ __forceinline__ void run(double2* u, int s) {
-		const double c[4] = {1.0, 0.62348980185873353053, -0.22252093395631440429, -0.90096886790241912624};
-		const double sn[4] = {0.0, 0.78183148246802980871, 0.97492791218182360702, 0.43388373911755812048};
-		double2 a[4], b[4];
-		#pragma unroll
-		for (int q = 1; q < 4; q++) { a[q] = cadd(u[q], u[7 - q]); b[q] = csub(u[q], u[7 - q]); }
-		const double2 x0 = u[0];
-		u[0] = cadd(x0, cadd(a[1], cadd(a[2], a[3])));
-		#pragma unroll
-		for (int k = 1; k < 4; k++) {
-			double2 r = x0, im = make_double2(0.0, 0.0);
-			#pragma unroll
-			for (int q = 1; q < 4; q++) {
-				const int j = (q * k) % 7;
-				const double cq = (j < 4) ? c[j] : c[7 - j];
-				const double sq = (j < 4) ? sn[j] : -sn[7 - j];
-				r.x = fma(cq, a[q].x, r.x);  r.y = fma(cq, a[q].y, r.y);
-				im.x = fma(sq, b[q].x, im.x); im.y = fma(sq, b[q].y, im.y);
-			}
-			// y_k = r + i s im,  y_{7-k} = r - i s im
-			const double2 t = make_double2(-s * im.y, s * im.x);
-			u[k] = cadd(r, t);
-			u[7 - k] = csub(r, t);
-		}
-	}
-};
-
-// Shared-memory layout: element i of sequence s lives at s*seq + i + i/8.
-// The pad of one slot per 8 elements spreads the stride-R writes of the first
-// Stockham pass over the banks, and seq = 2 mod 8 (in 16-byte units) spreads
-// the S sequences, so both the passes and the latitude-pair loads/stores are
-// free of bank conflicts.
-__device__ __forceinline__ int sidx(int s, int i, int seq) { return s * seq + i + (i >> 3); }
-
-// q = x / d, r = x % d for 0 <= x < 2^22 with a float reciprocal and one
-// correction step (avoids the integer division sequence in the inner loops).
-__device__ __forceinline__ void divmod(int x, int d, float inv, int& q, int& r)
-{
-	q = __float2int_rz(__int2float_rn(x) * inv);
-	r = x - q * d;
-	if (r < 0) { q--; r += d; }
-	else if (r >= d) { q++; r -= d; }
-}
-
-// One Stockham pass of radix R over S sequences of length N, from X to Y.
-// Butterfly b of a sequence reads element b + q*N/R (q < R), applies twiddles
-// w^{q*k*N/(p*R)} with k = b mod p, runs the R-point DFT and writes element
-// (b - k)*R + k + q*p.
-template <int R>
-__device__ __forceinline__ void fft_pass(const double2* __restrict__ X, double2* __restrict__ Y, int N, int S, int seq,
-                                         int p, const double2* __restrict__ tw, int sign)
-{
-	const int nbf = N / R;
-	const int total = S * nbf;
-	const int tstep = N / (p * R);
-	const float inv_nbf = 1.0f / nbf, inv_p = 1.0f / p;
-	for (int g = threadIdx.x; g < total; g += blockDim.x) {
-		int sq, b, q0, k;
-		divmod(g, nbf, inv_nbf, sq, b);
-		divmod(b, p, inv_p, q0, k);
-		double2 u[R];
-		#pragma unroll
-		for (int q = 0; q < R; q++) u[q] = X[sidx(sq, b + q * nbf, seq)];
-		if (k) {
-			// w^q by repeated multiplication from one table entry (error ~q ulp)
-			double2 w1 = __ldg(tw + k * tstep);
-			if (sign < 0) w1.y = -w1.y;
-			double2 w = w1;
-			#pragma unroll
-			for (int q = 1; q < R; q++) {
-				u[q] = cmul(u[q], w);
-				if (q + 1 < R) w = cmul(w, w1);
-			}
-		}
-		Dft<R>::run(u, sign);
-		const int o = (b - k) * R + k;
-		#pragma unroll
-		for (int q = 0; q < R; q++) Y[sidx(sq, o + q * p, seq)] = u[q];
-	}
-	__syncthreads();
-}
-
-// Runs all passes; returns the buffer (X or Y) that holds the result.
-__device__ __forceinline__ double2* fft_run(double2* X, double2* Y, int N, int S, int seq, unsigned long long rcode,
-                                            int nradix, const double2* __restrict__ tw, int sign)
-{
-	int pp = 1;
-	for (int r = 0; r < nradix; r++) {
-		const int R = (int)((rcode >> (4 * r)) & 15);
-		switch (R) {
-			case 8: fft_pass<8>(X, Y, N, S, seq, pp, tw, sign); break;
-			case 4: fft_pass<4>(X, Y, N, S, seq, pp, tw, sign); break;
-			case 2: fft_pass<2>(X, Y, N, S, seq, pp, tw, sign); break;
-			case 3: fft_pass<3>(X, Y, N, S, seq, pp, tw, sign); break;
-			case 5: fft_pass<5>(X, Y, N, S, seq, pp, tw, sign); break;
-			default: fft_pass<7>(X, Y, N, S, seq, pp, tw, sign); break;
-		}
-		pp *= R;
-		double2* t = X; X = Y; Y = t;
-	}
-	return X;
-}
-
-__device__ __forceinline__ int seq_len(int N, int S)
-{
-	const int a = N + (N >> 3);
-	return a + (((S >= 8 ? 1 : 8 / S) - a) & 7);
-}
-
-// Synthesis: F[fc][m][theta] (m <= mlim) -> spatial field-component fc.
-// Sequence s of the CTA packs latitudes lat0+2s (real part) and lat0+2s+1
-// (imaginary part): Z_k = A_k + i B_k, Z_{N-k} = conj(A_k) + i conj(B_k).
-template <int S>
-__global__ void __launch_bounds__(768) fft_synth_kernel(FftParams p)
-{
-	extern __shared__ double2 smem[];
-	const int N = p.N, T = blockDim.x, seq = seq_len(N, S);
-	double2* X = smem;
-	double2* Y = smem + S * seq;
-	const int fc = blockIdx.y;
-	const int lat0 = blockIdx.x * 2 * S;
-	const double2* Ff = p.F + (long)fc * p.fstride;
-	const int ml = p.mlim;
-	// zero the band between +mlim and -mlim
-	const int nz = N - 2 * ml - 1;
-	for (int e = threadIdx.x; e < S * nz; e += T) {
-		const int s = e / nz, i = ml + 1 + (e - s * nz);
-		X[sidx(s, i, seq)] = make_double2(0.0, 0.0);
-	}
-	const int nload = (ml + 1) * S;
-	for (int e0 = threadIdx.x; e0 < nload; e0 += 4 * T) {
-		double2 a[4], b[4];
-		#pragma unroll
-		for (int u = 0; u < 4; u++) {
-			const int e = e0 + u * T;
-			const int k = e / S, s = e - k * S;
-			const int ra = lat0 + 2 * s;
-			a[u] = make_double2(0.0, 0.0); b[u] = make_double2(0.0, 0.0);
-			if (e < nload && ra < p.nlat) {
-				a[u] = __ldg(Ff + (long)k * p.nlat + ra);
-				b[u] = __ldg(Ff + (long)k * p.nlat + ra + 1);
-			}
-		}
-		#pragma unroll
-		for (int u = 0; u < 4; u++) {
-			const int e = e0 + u * T;
-			if (e >= nload) continue;
-			const int k = e / S, s = e - k * S;
-			if (k == 0) { a[u].y = 0.0; b[u].y = 0.0; }
-			X[sidx(s, k, seq)] = make_double2(a[u].x - b[u].y, a[u].y + b[u].x);
-			if (k > 0) X[sidx(s, N - k, seq)] = make_double2(a[u].x + b[u].y, b[u].x - a[u].y);
-		}
-	}
-	__syncthreads();
-	X = fft_run(X, Y, N, S, seq, p.rcode, p.nradix, p.tw, +1);
-	const int c = fc / p.nf;
-	double* out = (c == 0 ? p.spat[0] : c == 1 ? p.spat[1] : p.spat[2]) + (long)(fc - c * p.nf) * p.spat_dist;
-	if (!p.phi_contiguous) {
-		for (int e = threadIdx.x; e < N * S; e += T) {
-			const int j = e / S, s = e - j * S;
-			const int row = lat0 + 2 * s;
-			if (row < p.nlat) {
-				const double2 z = X[sidx(s, j, seq)];
-				double* o = out + (long)j * p.nlat + row;
-				if (p.vec2) *reinterpret_cast<double2*>(o) = z;
-				else { o[0] = z.x; o[1] = z.y; }
-			}
-		}
-	} else {
-		for (int e = threadIdx.x; e < N * S; e += T) {
-			const int s = e / N, j = e - s * N;
-			const int row = lat0 + 2 * s;
-			if (row < p.nlat) {
-				const double2 z = X[sidx(s, j, seq)];
-				out[(long)row * N + j] = z.x;
-				out[(long)(row + 1) * N + j] = z.y;
-			}
-		}
-	}
-}
-
-// Analysis: spatial field-component fc -> F[fc][m][theta] = A_m / N for m <= mlim,
-// with A_k = (Z_k + conj Z_{N-k})/2 and B_k = (Z_k - conj Z_{N-k})/(2i).
-template <int S>
-__global__ void __launch_bounds__(768) fft_analys_kernel(FftParams p)
-{
-	extern __shared__ double2 smem[];
-	const int N = p.N, T = blockDim.x, seq = seq_len(N, S);
-	double2* X = smem;
-	double2* Y = smem + S * seq;
-	const int fc = blockIdx.y;
-	const int lat0 = blockIdx.x * 2 * S;
-	const int c = fc / p.nf;
-	const double* in = (c == 0 ? p.spat_in[0] : c == 1 ? p.spat_in[1] : p.spat_in[2]) + (long)(fc - c * p.nf) * p.spat_dist;
-	if (!p.phi_contiguous) {
-		// 8 independent loads in flight per thread before the shared-memory stores
-		for (int e0 = threadIdx.x; e0 < N * S; e0 += 8 * T) {
-			double2 v[8];
-			#pragma unroll
-			for (int u = 0; u < 8; u++) {
-				const int e = e0 + u * T;
-				const int j = e / S, s = e - j * S;
-				const int row = lat0 + 2 * s;
-				v[u] = make_double2(0.0, 0.0);
-				if (e < N * S && row < p.nlat) {
-					const double* i0 = in + (long)j * p.nlat + row;
-					v[u] = p.vec2 ? __ldg(reinterpret_cast<const double2*>(i0)) : make_double2(__ldg(i0), __ldg(i0 + 1));
-				}
-			}
-			#pragma unroll
-			for (int u = 0; u < 8; u++) {
-				const int e = e0 + u * T;
-				if (e < N * S) { const int j = e / S, s = e - j * S; X[sidx(s, j, seq)] = v[u]; }
-			}
-		}
-	} else {
-		for (int e = threadIdx.x; e < N * S; e += T) {
-			const int s = e / N, j = e - s * N;
-			const int row = lat0 + 2 * s;
-			double2 v = make_double2(0.0, 0.0);
-			if (row < p.nlat) v = make_double2(in[(long)row * N + j], in[(long)(row + 1) * N + j]);
-			X[sidx(s, j, seq)] = v;
-		}
-	}
-	__syncthreads();
-	X = fft_run(X, Y, N, S, seq, p.rcode, p.nradix, p.tw, -1);
-	double2* Ff = p.F + (long)fc * p.fstride;
-	const double sc = 0.5 / N;
-	for (int e = threadIdx.x; e < (p.mlim + 1) * S; e += T) {
-		const int k = e / S, s = e - k * S;
-		const int ra = lat0 + 2 * s;
-		const double2 z = X[sidx(s, k, seq)];
-		const double2 w = X[sidx(s, k ? N - k : 0, seq)];
-		if (ra < p.nlat) {
-			Ff[(long)k * p.nlat + ra] = make_double2(sc * (z.x + w.x), sc * (z.y - w.y));
-			Ff[(long)k * p.nlat + ra + 1] = make_double2(sc * (z.y + w.y), -sc * (z.x - w.x));
-		}
-	}
-}
+using namespace shtb_dft;
+using namespace shtb_fft_tma;
+using namespace shtb_fft_grid;
 
 // ===========================================================================
 // Fused kernels for nphi = 3 * 2^k (192 ... 6144), the sizes of Gauss grids
@@ -546,7 +237,7 @@ __device__ __forceinline__ void fused_fft(double2* X, const double2* tw, int sig
 	Chain<N, S, R0, MODE, Rest...>::run(X, tw, sign, st, tid);
 }
 
-template <int N, int S>
+template <int N, int S, class G>
 __global__ void __launch_bounds__(Geo<N, S>::T) fft3_synth_kernel(FftParams p)
 {
 	extern __shared__ double2 smem[];
@@ -563,24 +254,22 @@ __global__ void __launch_bounds__(Geo<N, S>::T) fft3_synth_kernel(FftParams p)
 		return (j <= ml) ? make_double2(a.x - b.y, a.y + b.x) : make_double2(a.x + b.y, b.x - a.y);
 	};
 	const int c = fc / p.nf;
-	double* out = (c == 0 ? p.spat[0] : c == 1 ? p.spat[1] : p.spat[2]) + (long)(fc - c * p.nf) * p.spat_dist;
+	G* out = grid_out<G>(p, c, fc);
 	const bool phi = p.phi_contiguous, v2 = p.vec2;
 	auto st = [&](int s, int j, double2 z) {
 		const int row = lat0 + 2 * s;
 		if (row >= nlat) return;
 		if (!phi) {
-			double* o = out + (long)j * nlat + row;
-			if (v2) *reinterpret_cast<double2*>(o) = z;
-			else { o[0] = z.x; o[1] = z.y; }
+			store_pair(out + (long)j * nlat + row, z, v2);
 		} else {
-			out[(long)row * N + j] = z.x;
-			out[(long)(row + 1) * N + j] = z.y;
+			out[(long)row * N + j] = (G) z.x;
+			out[(long)(row + 1) * N + j] = (G) z.y;
 		}
 	};
 	fused_fft<N, S, true>(smem, p.tw, +1, ld, st, NoHook{}, threadIdx.x, typename NphiPlan<N>::L{});
 }
 
-template <int N, int S>
+template <int N, int S, class G>
 __global__ void __launch_bounds__(Geo<N, S>::T) fft3_analys_kernel(FftParams p)
 {
 	extern __shared__ double2 smem[];
@@ -588,15 +277,12 @@ __global__ void __launch_bounds__(Geo<N, S>::T) fft3_analys_kernel(FftParams p)
 	const int lat0 = blockIdx.x * 2 * S;
 	const int nlat = p.nlat;
 	const int c = fc / p.nf;
-	const double* in = (c == 0 ? p.spat_in[0] : c == 1 ? p.spat_in[1] : p.spat_in[2]) + (long)(fc - c * p.nf) * p.spat_dist;
+	const G* in = grid_in<G>(p, c, fc);
 	const bool phi = p.phi_contiguous, v2 = p.vec2;
 	auto ld = [&](int s, int j) -> double2 {
 		const int row = lat0 + 2 * s;
 		if (row >= nlat) return make_double2(0.0, 0.0);
-		if (!phi) {
-			const double* i0 = in + (long)j * nlat + row;
-			return v2 ? __ldg(reinterpret_cast<const double2*>(i0)) : make_double2(__ldg(i0), __ldg(i0 + 1));
-		}
+		if (!phi) return load_pair(in + (long)j * nlat + row, v2);
 		return make_double2(__ldg(in + (long)row * N + j), __ldg(in + (long)(row + 1) * N + j));
 	};
 	// Fourier rows straight from the last radix pass (pairs z_k, z_{N-k})
@@ -778,40 +464,7 @@ struct TmaTiles {
 	int v4;           // F rows 32-byte aligned at even latitudes: one 32-byte store per latitude pair
 };
 
-constexpr uint64_t FT_WAIT_NS = 1000000000ull;   // time limit of every mbarrier wait
-
 __device__ int g_fft_wait_err;                    // set when a bounded wait gave up
-
-__device__ __forceinline__ uint32_t su32(const void* ptr) { return static_cast<uint32_t>(__cvta_generic_to_shared(ptr)); }
-
-__device__ __forceinline__ uint64_t gtimer()
-{
-	uint64_t t;
-	asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-	return t;
-}
-
-__device__ __forceinline__ bool fbar_wait(uint64_t* bar, uint32_t parity)
-{
-	const uint32_t a = su32(bar);
-	const uint64_t t0 = gtimer();
-	for (int it = 0;; it++) {
-		if ((it & 1023) == 1023 && gtimer() - t0 > FT_WAIT_NS) return false;
-		uint32_t done;
-		asm volatile("{\n\t.reg .pred p;\n\t"
-		             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-		             "selp.u32 %0, 1, 0, p;\n\t}"
-		             : "=r"(done) : "r"(a), "r"(parity) : "memory");
-		if (done) return true;
-	}
-}
-
-__device__ __forceinline__ void tma_tile3(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar)
-{
-	asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-	             :: "r"(su32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(su32(bar))
-	             : "memory");
-}
 
 // One thread: announce the bytes of a tile, then issue its box copies
 // (latitude coordinate c0, rows c * box, field c2).
@@ -871,7 +524,7 @@ __device__ __forceinline__ void store_tile(const CUtensorMap* map, const char* X
 
 // TOUT: theta-contiguous output written by tensor stores of whole tiles
 // (rows of 2 S latitudes) from X, instead of 16-byte stores per latitude pair
-template <int N, int S, bool TOUT>
+template <int N, int S, bool TOUT, class G>
 __global__ void __launch_bounds__(Geo<N, S>::T, 768 / Geo<N, S>::T) fft4_synth_kernel(
 	const __grid_constant__ CUtensorMap fmap, const __grid_constant__ CUtensorMap o0, const __grid_constant__ CUtensorMap o1,
 	const __grid_constant__ CUtensorMap o2, FftParams p, TmaTiles tt)
@@ -928,18 +581,16 @@ __global__ void __launch_bounds__(Geo<N, S>::T, 768 / Geo<N, S>::T) fft4_synth_k
 			const CUtensorMap* om = (c == 0) ? &o0 : (c == 1 ? &o1 : &o2);
 			store_tile(om, base, N / BJ, BJ, BJ * S * 16, lat0, fc - c * p.nf);
 		} else {
-			double* out = (c == 0 ? p.spat[0] : c == 1 ? p.spat[1] : p.spat[2]) + (long)(fc - c * p.nf) * p.spat_dist;
+			G* out = grid_out<G>(p, c, fc);
 			const bool phi = p.phi_contiguous, v2 = p.vec2;
 			auto st = [&](int s, int j, double2 z) {
 				const int row = lat0 + 2 * s;
 				if (row >= nlat) return;
 				if (!phi) {
-					double* o = out + (long)j * nlat + row;
-					if (v2) *reinterpret_cast<double2*>(o) = z;
-					else { o[0] = z.x; o[1] = z.y; }
+					store_pair(out + (long)j * nlat + row, z, v2);
 				} else {
-					out[(long)row * N + j] = z.x;
-					out[(long)(row + 1) * N + j] = z.y;
+					out[(long)row * N + j] = (G) z.x;
+					out[(long)(row + 1) * N + j] = (G) z.y;
 				}
 			};
 			fused_fft<N, S, 1>(X, p.tw, +1, ld, st, prefetch, threadIdx.x, typename NphiPlan<N>::L{});
@@ -948,20 +599,19 @@ __global__ void __launch_bounds__(Geo<N, S>::T, 768 / Geo<N, S>::T) fft4_synth_k
 	if (TOUT && threadIdx.x == 0) store_reads_done();
 }
 
-template <int N, int S>
+template <int N, int S, class G>
 __global__ void __launch_bounds__(Geo<N, S>::T, 768 / Geo<N, S>::T) fft4_analys_kernel(
 	const __grid_constant__ CUtensorMap m0, const __grid_constant__ CUtensorMap m1, const __grid_constant__ CUtensorMap m2,
 	FftParams p, TmaTiles tt)
 {
-	using G = Geo<N, S>;
 	extern __shared__ __align__(128) char fsm[];
 	__shared__ __align__(8) uint64_t bar;
 	char* base = fsm + ((128u - (su32(fsm) & 127u)) & 127u);   // tensor copies land on 128-byte boundaries
 	double2* X = reinterpret_cast<double2*>(base);
 	char* stage = base + tt.stage_off;
-	const double* stg = reinterpret_cast<const double*>(stage);
+	const G* stg = reinterpret_cast<const G*>(stage);
 	const int nlat = p.nlat, nf = p.nf;
-	const int box_bytes = box_j(N) * 2 * S * 8;
+	const int box_bytes = box_j(N) * 2 * S * sizeof(G);
 	auto issue = [&](int t) {
 		const int fc = t / tt.nlg, c = fc / nf;
 		const CUtensorMap* m = (c == 0) ? &m0 : (c == 1 ? &m1 : &m2);
@@ -976,7 +626,10 @@ __global__ void __launch_bounds__(Geo<N, S>::T, 768 / Geo<N, S>::T) fft4_analys_
 		const int lat0 = (tile - fc * tt.nlg) * 2 * S;
 		int rs = 2 * S;                         // opaque per tile, as mlim in the synthesis
 		asm volatile("" : "+r"(rs));
-		auto ld = [&](int s, int j) -> double2 { return *reinterpret_cast<const double2*>(stg + j * rs + 2 * s); };
+		auto ld = [&](int s, int j) -> double2 {
+			const typename Pair<G>::T v = *reinterpret_cast<const typename Pair<G>::T*>(stg + j * rs + 2 * s);
+			return make_double2(v.x, v.y);
+		};
 		const int next = tile + gridDim.x;
 		auto prefetch = [&]() {
 			if (threadIdx.x == 0 && next < tt.ntiles) {
@@ -1004,37 +657,6 @@ __global__ void __launch_bounds__(Geo<N, S>::T, 768 / Geo<N, S>::T) fft4_analys_
 	}
 }
 
-// the driver's tensor-map encoder, resolved once (thread-safe static initialisation)
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
-{
-	static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
-		void* f = nullptr;
-		cudaDriverEntryPointQueryResult q;
-		if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-		    q == cudaDriverEntryPointSuccess)
-			return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
-		cudaGetLastError();
-		return (PFN_cuTensorMapEncodeTiled_v12000) nullptr;
-	}();
-	return fn;
-}
-
-// 3-d FP64 tensor map, dims / byte strides of dims 1 and 2 / box, no swizzle,
-// zero fill out of range
-bool encode3(CUtensorMap* m, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1, uint64_t s2,
-             uint32_t b0, uint32_t b1)
-{
-	PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-	if (!enc || ((uintptr_t) base & 15) || (s1 & 15) || (s2 & 15) || ((b0 * 8) & 15)) return false;
-	const cuuint64_t dims[3] = {d0, d1, d2};
-	const cuuint64_t strides[2] = {s1, s2};
-	const cuuint32_t box[3] = {b0, b1, 1};
-	const cuuint32_t es[3] = {1, 1, 1};
-	return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<void*>(base), dims, strides, box, es,
-	           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-	           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 int sm_count()
 {
 	static const int n = [] {
@@ -1055,7 +677,8 @@ bool f_map(CUtensorMap* m, const FftParams& p, int nfc, int S, int box)
 // theta-contiguous spatial component c: dims (nlat, nphi, fields)
 bool grid_map(CUtensorMap* m, const double* base, const FftParams& p, int N, int S)
 {
-	return encode3(m, base, p.nlat, N, p.nf, 8 * (uint64_t) p.nlat, 8 * (uint64_t) p.spat_dist, 2 * S, box_j(N));
+	const uint64_t e = p.f32 ? 4 : 8;
+	return encode3(m, base, p.nlat, N, p.nf, e * p.nlat, e * p.spat_dist, 2 * S, box_j(N), p.f32);
 }
 
 template <int N, int S>
@@ -1079,7 +702,7 @@ bool launch_fft4(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 		tt.ncopy = (rows + tt.box - 1) / tt.box;
 		stage_bytes = (size_t) tt.ncopy * tt.box * 2 * S * 16;
 		if (!f_map(&maps[0], p, nfc, S, tt.box)) return false;
-		tout = grid_ok && tstore;
+		tout = grid_ok && tstore && !p.f32;
 		for (int c = 0; c < 3 && tout; c++) tout = grid_map(&maps[1 + c], p.spat[c < ncomp ? c : 0], p, N, S);
 	} else {
 		// theta-contiguous grids only (phi-contiguous rows are read faster
@@ -1087,7 +710,7 @@ bool launch_fft4(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 		if (!grid_ok) return false;
 		tt.box = box_j(N);
 		tt.ncopy = N / tt.box;
-		stage_bytes = (size_t) N * 2 * S * 8;
+		stage_bytes = (size_t) N * 2 * S * (p.f32 ? 4 : 8);
 		for (int c = 0; c < 3; c++)
 			if (!grid_map(&maps[c], p.spat_in[c < ncomp ? c : 0], p, N, S)) return false;
 	}
@@ -1096,21 +719,29 @@ bool launch_fft4(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 	tt.stage_off = (int)(((size_t) S * G::SEQ * sizeof(double2) + 127) / 128 * 128);
 	const size_t smem = tt.stage_off + stage_bytes + 128;
 	if (smem > 226 * 1024) return false;
-	const void* fn = synth ? (tout ? (const void*) fft4_synth_kernel<N, S, true> : (const void*) fft4_synth_kernel<N, S, false>)
-	                       : (const void*) fft4_analys_kernel<N, S>;
-	int per_sm = 0;
-	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, G::T, smem) != cudaSuccess || per_sm <= 0) {
-		cudaGetLastError();
-		return false;
-	}
-	const int grid = std::min(tt.ntiles, per_sm * sm_count());
-	if (synth) {
-		if (tout) fft4_synth_kernel<N, S, true><<<grid, G::T, smem, st>>>(maps[0], maps[1], maps[2], maps[3], p, tt);
-		else fft4_synth_kernel<N, S, false><<<grid, G::T, smem, st>>>(maps[0], maps[0], maps[0], maps[0], p, tt);
-	} else {
-		fft4_analys_kernel<N, S><<<grid, G::T, smem, st>>>(maps[0], maps[1], maps[2], p, tt);
-	}
-	return true;
+	auto go = [&](auto kern) {
+		// the occupancy of the thread's last kernel and size is kept: the query costs about as much as a launch
+		static thread_local const void* last_fn = nullptr;
+		static thread_local size_t last_smem = 0;
+		static thread_local int per_sm = 0;
+		if (last_fn != (const void*) kern || last_smem != smem) {
+			last_fn = nullptr;
+			if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, G::T, smem) != cudaSuccess || per_sm <= 0) {
+				cudaGetLastError();
+				return false;
+			}
+			last_fn = (const void*) kern; last_smem = smem;
+		}
+		const int grid = std::min(tt.ntiles, per_sm * sm_count());
+		if constexpr (std::is_same_v<decltype(kern), decltype(&fft4_analys_kernel<N, S, double>)>)
+			kern<<<grid, G::T, smem, st>>>(maps[0], maps[1], maps[2], p, tt);
+		else
+			kern<<<grid, G::T, smem, st>>>(maps[0], maps[tout ? 1 : 0], maps[tout ? 2 : 0], maps[tout ? 3 : 0], p, tt);
+		return true;
+	};
+	if (synth) return p.f32 ? go(fft4_synth_kernel<N, S, false, float>)
+	                        : (tout ? go(fft4_synth_kernel<N, S, true, double>) : go(fft4_synth_kernel<N, S, false, double>));
+	return p.f32 ? go(fft4_analys_kernel<N, S, float>) : go(fft4_analys_kernel<N, S, double>);
 }
 
 template <int N, int S>
@@ -1119,8 +750,9 @@ bool launch_fft3(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 	using G = Geo<N, S>;
 	const size_t smem = sizeof(double2) * (size_t) S * G::SEQ;
 	dim3 grid((p.nlat + 2 * S - 1) / (2 * S), nfc);
-	if (synth) fft3_synth_kernel<N, S><<<grid, G::T, smem, st>>>(p);
-	else fft3_analys_kernel<N, S><<<grid, G::T, smem, st>>>(p);
+	auto go = [&](auto kern) { kern<<<grid, G::T, smem, st>>>(p); };
+	if (p.f32) go(synth ? fft3_synth_kernel<N, S, float> : fft3_analys_kernel<N, S, float>);
+	else go(synth ? fft3_synth_kernel<N, S, double> : fft3_analys_kernel<N, S, double>);
 	return true;
 }
 
@@ -1160,23 +792,18 @@ bool launch_fft4_n(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 	}
 }
 
-// four-step path: nphi = 12288 on theta-contiguous grids with 16-byte
-// aligned latitude pairs and (analysis) a scratch grid; false otherwise
+// four-step path on theta-contiguous grids with 16-byte aligned latitude pairs
+// and (analysis) a scratch grid; false otherwise.
+template <int N1, int N2>
 bool launch_fourstep(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 {
-	constexpr int N1 = 96, N2 = 128;
-	if (p.N != N1 * N2 || p.phi_contiguous || !p.vec2 || !p.tw1 || p.generic != 0 || (!synth && !p.scratch)) return false;
+	if (p.N != N1 * N2 || p.phi_contiguous || !p.vec2 || !p.tw1 || p.generic != 0 || p.f32 || (!synth && !p.scratch)) return false;
 	if (p.nlat % 2 || ((uintptr_t) p.F & 31)) return false;
 	using G1 = Geo<N1, FS_S>;
 	using G2 = Geo<N2, FS_S>;
 	using G3 = Geo<N1, 2 * FS_S>;
 	const size_t s1 = sizeof(double2) * (size_t) FS_S * G1::SEQ, s2 = sizeof(double2) * (size_t) FS_S * G2::SEQ;
 	const size_t s3 = sizeof(double2) * (size_t)(2 * FS_S) * G3::SEQ;
-	static bool attr = false;
-	if (!attr) {
-		cudaFuncSetAttribute(fft_fs_analys2_kernel<N1, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) s3);
-		attr = true;
-	}
 	const int nlb = (p.nlat + 2 * FS_S - 1) / (2 * FS_S);
 	if (synth) {
 		fft_fs_synth1_kernel<N1, N2><<<dim3(nlb, N2, nfc), G1::T, s1, st>>>(p);
@@ -1189,9 +816,16 @@ bool launch_fourstep(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 	return true;
 }
 
+template <int N1, int N2>
+void set_fourstep_limits()
+{
+	cudaFuncSetAttribute(fft_fs_analys2_kernel<N1, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                     (int)(sizeof(double2) * 2 * FS_S * Geo<N1, 2 * FS_S>::SEQ));
+}
+
 bool launch_fused(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 {
-	if (launch_fourstep(p, nfc, st, synth)) return true;
+	if (launch_fourstep<96, 128>(p, nfc, st, synth)) return true;
 	if (p.generic == 0 || p.generic == 3) {
 		bool done = false;
 		switch (p.N) {
@@ -1220,9 +854,22 @@ bool launch_fused(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 template <int N, int S>
 void set_fft4_limits(int lim)
 {
-	cudaFuncSetAttribute(fft4_synth_kernel<N, S, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-	cudaFuncSetAttribute(fft4_synth_kernel<N, S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-	cudaFuncSetAttribute(fft4_analys_kernel<N, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+	auto set = [&](auto kern) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, lim); };
+	set(fft4_synth_kernel<N, S, true, double>);
+	set(fft4_synth_kernel<N, S, false, double>);
+	set(fft4_synth_kernel<N, S, false, float>);
+	set(fft4_analys_kernel<N, S, double>);
+	set(fft4_analys_kernel<N, S, float>);
+}
+
+template <int N, int S>
+void set_fft3_limits(int lim)
+{
+	auto set = [&](auto kern) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, lim); };
+	set(fft3_synth_kernel<N, S, double>);
+	set(fft3_synth_kernel<N, S, float>);
+	set(fft3_analys_kernel<N, S, double>);
+	set(fft3_analys_kernel<N, S, float>);
 }
 
 template <int N>
@@ -1236,19 +883,15 @@ void set_fused_limits()
 		if constexpr (2 * N / 8 <= 768) set_fft4_limits<N, 2>(lim4);
 		if constexpr (4 * N / 8 <= 768) set_fft4_limits<N, 4>(lim4);
 	}
-	cudaFuncSetAttribute(fft3_synth_kernel<N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-	cudaFuncSetAttribute(fft3_analys_kernel<N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+	set_fft3_limits<N, 1>(lim);
 	if constexpr (2 * N / 8 <= 768) {
-		cudaFuncSetAttribute(fft3_synth_kernel<N, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-		cudaFuncSetAttribute(fft3_analys_kernel<N, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+		set_fft3_limits<N, 2>(lim);
 	}
 	if constexpr (4 * N / 8 <= 768) {
-		cudaFuncSetAttribute(fft3_synth_kernel<N, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-		cudaFuncSetAttribute(fft3_analys_kernel<N, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+		set_fft3_limits<N, 4>(lim);
 	}
 	if constexpr (8 * (N + (N >> 3) + 1) * 16 <= 227 * 1024) {
-		cudaFuncSetAttribute(fft3_synth_kernel<N, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-		cudaFuncSetAttribute(fft3_analys_kernel<N, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+		set_fft3_limits<N, 8>(lim);
 	}
 }
 
@@ -1260,18 +903,9 @@ static int seq_len_host(int N, int S)
 	return a + (((S >= 8 ? 1 : 8 / S) - a) & 7);
 }
 
-int fft_threads(int N, int S, unsigned long long rcode, int nradix)
-{
-	(void) rcode; (void) nradix;
-	// about one radix-8 butterfly per thread
-	int T = (S * N / 8 + 31) / 32 * 32;
-	return T < 64 ? 64 : (T > 768 ? 768 : T);
-}
-
 size_t fft_smem_bytes(int N, int S) { return 2 * sizeof(double2) * (size_t) S * seq_len_host(N, S); }
 
-// sizes with a fused pass chain (one in-place buffer: these may exceed the
-// generic kernels' two-buffer limit)
+// sizes with a fused pass chain (these may exceed the generic kernels' limit)
 bool fft_fused_available(int N)
 {
 	switch (N) {
@@ -1289,14 +923,7 @@ void launch_fft_synth(const FftParams& p, int nfc, cudaStream_t st)
 	g_fft4_ran = false;
 	if (p.generic != 1 && launch_fused(p, nfc, st, true)) { g_last_fft_path = g_fft4_ran ? 2 : 1; shtb_count_launch(); return; }
 	g_last_fft_path = 0;
-	const int T = fft_threads(p.N, p.S, p.rcode, p.nradix);
-	const size_t smem = fft_smem_bytes(p.N, p.S);
-	dim3 grid((p.nlat + 2 * p.S - 1) / (2 * p.S), nfc);
-	switch (p.S) {
-		case 4: fft_synth_kernel<4><<<grid, T, smem, st>>>(p); break;
-		case 2: fft_synth_kernel<2><<<grid, T, smem, st>>>(p); break;
-		default: fft_synth_kernel<1><<<grid, T, smem, st>>>(p); break;
-	}
+	launch_fft_gen(p, nfc, st, true);
 	shtb_count_launch();
 }
 
@@ -1305,30 +932,25 @@ void launch_fft_analys(const FftParams& p, int nfc, cudaStream_t st)
 	g_fft4_ran = false;
 	if (p.generic != 1 && launch_fused(p, nfc, st, false)) { g_last_fft_path = g_fft4_ran ? 2 : 1; shtb_count_launch(); return; }
 	g_last_fft_path = 0;
-	const int T = fft_threads(p.N, p.S, p.rcode, p.nradix);
-	const size_t smem = fft_smem_bytes(p.N, p.S);
-	dim3 grid((p.nlat + 2 * p.S - 1) / (2 * p.S), nfc);
-	switch (p.S) {
-		case 4: fft_analys_kernel<4><<<grid, T, smem, st>>>(p); break;
-		case 2: fft_analys_kernel<2><<<grid, T, smem, st>>>(p); break;
-		default: fft_analys_kernel<1><<<grid, T, smem, st>>>(p); break;
-	}
+	launch_fft_gen(p, nfc, st, false);
 	shtb_count_launch();
+}
+
+// nphi = n1 n2 of the four-step kernels
+bool fft_fourstep_factors(int N, int& n1, int& n2)
+{
+	if (N == 12288) { n1 = 96; n2 = 128; return true; }
+	return false;
 }
 
 void fft_set_smem_limits()
 {
+	set_fourstep_limits<96, 128>();
 	tensor_map_encoder();    // resolved here, outside any stream capture
 	sm_count();
 	set_fused_limits<192>(); set_fused_limits<384>(); set_fused_limits<768>();
 	set_fused_limits<1536>(); set_fused_limits<3072>(); set_fused_limits<6144>(); set_fused_limits<12288>();
-	const int lim = 227 * 1024;
-	cudaFuncSetAttribute(fft_synth_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-	cudaFuncSetAttribute(fft_synth_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-	cudaFuncSetAttribute(fft_synth_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-	cudaFuncSetAttribute(fft_analys_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-	cudaFuncSetAttribute(fft_analys_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-	cudaFuncSetAttribute(fft_analys_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+	fft_gen_set_smem_limits();
 }
 
 // Returns (and clears) the flag that a bounded wait of the prefetched FFT
@@ -1342,5 +964,5 @@ int fft_take_wait_error()
 		const int z = 0;
 		cudaMemcpyToSymbol(g_fft_wait_err, &z, sizeof(int));
 	}
-	return e;
+	return e | fft_gen_take_wait_error();
 }

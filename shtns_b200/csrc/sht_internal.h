@@ -22,8 +22,7 @@
 // pipeline stages (for shtns_b200_stage_times)
 #define SHTB_NSTAGES 6   // 0 prologue, 1 Legendre synthesis, 2 FFT synthesis, 3 FFT analysis, 4 Legendre analysis, 5 epilogue
 
-#define FFT_MAX_FACTORS 16
-#define FFT_NB 2      // butterflies held in registers per thread and pass
+#define FFT_MAX_PASSES 8
 
 // Per-order metadata, one entry per im = 0..mmax (int arrays on the device).
 struct MTables {
@@ -33,6 +32,15 @@ struct MTables {
 	int* voff;    // offset into per-degree vector coefficients (degrees m..lmax+1)
 	int* ckoff;   // first checkpoint segment of order im
 	int* tm;      // first theta row (north index) kept by the polar threshold
+};
+
+// Passes of the generic FFT kernels (sht_fft_gen.cu): radix, product of the
+// earlier radices, butterflies nphi / R, twiddle step nphi / (P R), 1 / P.
+struct FftPass { int R, P, nbf, ts; float inv_p; };
+struct FftGenPlan {
+	int np = 0;                          // passes (at least 2)
+	int E = 0;                           // complex values a thread holds: 12 or 16
+	FftPass ps[FFT_MAX_PASSES] = {};
 };
 
 // Public prefix must stay identical to shtns.h:struct shtns_info.
@@ -80,7 +88,8 @@ struct shtns_info {
 	int fft_generic;                     // FFT kernels: 0 automatic, 1 generic mixed-radix, 2 fused without prefetch, 3 no tensor stores
 	int fft_extra_tx;                    // test hook: bytes the prefetching FFT kernels expect beyond their copies (0)
 	int tile_wm;                         // Legendre tile shape option (0 automatic)
-	std::vector<int> fft_radix;          // factorisation of nphi
+	FftGenPlan fft_gen;                  // passes of the generic FFT kernels for nphi
+	FftGenPlan fft_gen_small;            // the same for calls of few latitudes (np = 0: none)
 	double Y00_1, Y10_ct, Y11_st;
 	// device tables
 	int dev;
@@ -89,7 +98,7 @@ struct shtns_info {
 	double *d_stdt_lo, *d_stdt_hi, *d_van_lo, *d_van_hi, *d_l2;
 	double2 *d_ck;                      // checkpoints (Y_k, Y_k+1), [segment][north row]
 	double2 *d_tw;                       // exp(+2 pi i j / nphi), j < nphi
-	double2 *d_tw4;                      // nphi = 12288: four-step factor tables (96 + 128 entries)
+	double2 *d_tw4;                      // four-step FFT sizes: factor tables (N1 + N2 entries)
 	double *d_fscr; size_t fscr_cap;     // four-step FFT analysis scratch (grow on demand)
 	MTables mt;
 	int *d_mint;                         // backing store of mt
@@ -214,8 +223,9 @@ struct PrepParams {
 };
 
 struct FftParams {
-	int N, S, nlat, mlim, nradix;
-	unsigned long long rcode;            // radices of nphi, 4 bits each, first pass in the low bits
+	int N, S, nlat, mlim;
+	int pairs;                           // latitude pairs per CTA asked for by the caller (0: automatic)
+	const FftGenPlan *gen, *gen_small;   // host pointers, read by the launchers only
 	const double2 *tw;
 	double2 *F;
 	long fstride;                        // complex elements between field-components in F
@@ -224,11 +234,12 @@ struct FftParams {
 	int nf;                              // fields per component
 	long spat_dist;
 	int phi_contiguous;
-	int vec2;                            // spatial pointers 16-byte aligned: latitude pairs moved as double2
+	int f32;                             // the spatial arrays are float (spat and spat_in point to floats)
+	int vec2;                            // latitude pairs of the spatial arrays aligned: moved as double2 (float2)
 	int extra_tx;                        // test hook: extra bytes expected per prefetched tile (0)
 	int generic;                         // 0 automatic, 1 generic mixed-radix kernels, 2 fused kernels without prefetch,
 	                                     // 3 prefetched loads with per-thread stores
-	const double2 *tw1, *tw2;            // four-step FFT (nphi = 96 x 128): exp(+2 pi i j / 96), exp(+2 pi i j / 128)
+	const double2 *tw1, *tw2;            // four-step FFT (nphi = N1 N2): exp(+2 pi i j / N1), exp(+2 pi i j / N2)
 	double *scratch;                     // four-step analysis: a grid per field-component (null: other kernels)
 };
 
@@ -270,9 +281,13 @@ void launch_leg_analys_simt(const LegParams& p, int kmax_all, cudaStream_t st);
 void free_split(shtns_cfg s);
 void launch_leg_multi(const LegParams* d_plist, const int4* d_work, int nwork, int* d_counter, int ckseg, bool synth,
                       int nctas, cudaStream_t st);
-int fft_threads(int N, int S, unsigned long long rcode, int nradix);
 bool fft_fused_available(int N);
+bool fft_fourstep_factors(int N, int& n1, int& n2);
 size_t fft_smem_bytes(int N, int S);
+bool fft_gen_plan(int N, FftGenPlan& g, int emax);
+void launch_fft_gen(const FftParams& p, int nfc, cudaStream_t st, bool synth);
+void fft_gen_set_smem_limits();
+int fft_gen_take_wait_error();
 void launch_fft_synth(const FftParams& p, int nfc, cudaStream_t st);
 void launch_fft_analys(const FftParams& p, int nfc, cudaStream_t st);
 int fft_take_wait_error();

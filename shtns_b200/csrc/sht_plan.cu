@@ -310,21 +310,13 @@ static double max_plm(shtns_cfg s, int im, long double x, long double sint)
 	return (double) v;
 }
 
-static int fft_factorize(int n, std::vector<int>& f)
+// nphi accepted by the FFT kernels: prime factors 2, 3, 5, 7, and either short
+// enough for a CTA's shared memory or one of the sizes with a fused chain
+static bool nphi_ok(int n)
 {
-	const int n0 = n;
-	f.clear();
-	while (n % 8 == 0) { f.push_back(8); n /= 8; }
-	while (n % 4 == 0) { f.push_back(4); n /= 4; }
-	while (n % 2 == 0) { f.push_back(2); n /= 2; }
-	while (n % 3 == 0) { f.push_back(3); n /= 3; }
-	while (n % 5 == 0) { f.push_back(5); n /= 5; }
-	while (n % 7 == 0) { f.push_back(7); n /= 7; }
-	int rmin = 8;
-	for (int r : f) rmin = r < rmin ? r : rmin;
-	(void) rmin;
-	// one CTA holds two padded buffers of a latitude pair in shared memory
-	return n == 1 && (int) f.size() <= FFT_MAX_FACTORS && (fft_smem_bytes(n0, 1) <= 227 * 1024 || fft_fused_available(n0));
+	int r = n;
+	for (int f : {2, 3, 5, 7}) while (r % f == 0) r /= f;
+	return r == 1 && (fft_smem_bytes(n, 1) <= 227 * 1024 || fft_fused_available(n));
 }
 
 // first checkpoint segment of every order for the current spacing s->ckseg
@@ -416,16 +408,13 @@ static int init_device(shtns_cfg s)
 	ok &= ok && shtb_cuda_ok(cudaMalloc(&s->d_mint, sizeof(int) * mi.size()), "order tables");
 	ok &= ok && shtb_cuda_ok(cudaMalloc(&s->d_tw, sizeof(double2) * tw.size()), "twiddles");
 	ok &= ok && shtb_cuda_ok(cudaMalloc(&s->d_ck, sizeof(double2) * ck_elems), "checkpoints");
-	if (ok && s->nphi == 12288) {
-		// factor tables of the four-step FFT, 12288 = 96 x 128
-		std::vector<double2> t4(96 + 128);
-		for (int j = 0; j < 96; j++) {
-			long double a = 2.0L * 3.14159265358979323846264338327950288L * j / 96.0L;
+	int f1, f2;
+	if (ok && fft_fourstep_factors(s->nphi, f1, f2)) {
+		// factor tables of the four-step FFT
+		std::vector<double2> t4(f1 + f2);
+		for (int j = 0; j < f1 + f2; j++) {
+			long double a = 2.0L * 3.14159265358979323846264338327950288L * (j < f1 ? (long double) j / f1 : (long double) (j - f1) / f2);
 			t4[j] = make_double2((double) std::cos(a), (double) std::sin(a));
-		}
-		for (int j = 0; j < 128; j++) {
-			long double a = 2.0L * 3.14159265358979323846264338327950288L * j / 128.0L;
-			t4[96 + j] = make_double2((double) std::cos(a), (double) std::sin(a));
 		}
 		ok &= shtb_cuda_ok(cudaMalloc(&s->d_tw4, sizeof(double2) * t4.size()), "FFT factor tables");
 		if (ok) cudaMemcpy(s->d_tw4, t4.data(), sizeof(double2) * t4.size(), cudaMemcpyHostToDevice);
@@ -515,8 +504,7 @@ extern "C" int shtns_set_grid_auto(shtns_cfg s, enum shtns_type flags, double ep
 	if (nl_order <= 0) nl_order = 1;
 	if (*nphi == 0) {
 		int n = (nl_order + 1) * s->mmax + 1;
-		std::vector<int> f;
-		while (!fft_factorize(n, f)) n++;
+		while (!nphi_ok(n)) n++;
 		*nphi = n;
 	}
 	if (*nlat == 0) {
@@ -529,11 +517,11 @@ extern "C" int shtns_set_grid_auto(shtns_cfg s, enum shtns_type flags, double ep
 	if (nl <= s->lmax) { plan_error("Nlat must be larger than Lmax"); return -1; }
 	if (np <= 2 * s->mmax) { plan_error("the sampling condition Nphi > 2*Mmax is not met."); return -1; }
 	if (nl > 65534 || np > 65534) { plan_error("Nlat or Nphi too large"); return -1; }
-	std::vector<int> rad;
-	if (!fft_factorize(np, rad)) { plan_error("Nphi must factor into 2, 3, 5 and 7 and not exceed 6400 (or be 3*2^k up to 12288)"); return -1; }
+	if (!nphi_ok(np)) { plan_error("Nphi must factor into 2, 3, 5 and 7 and not exceed 6400 (or be 3*2^k up to 12288)"); return -1; }
 	if (layout & SHT_PHI_CONTIGUOUS && layout & SHT_THETA_CONTIGUOUS) { plan_error("conflicting layout flags"); return -1; }
 	shtns_unset_grid(s);
-	s->fft_radix = rad;
+	fft_gen_plan(np, s->fft_gen_small, 8);
+	if (!fft_gen_plan(np, s->fft_gen, 16) && !fft_fused_available(np)) { plan_error("no FFT plan for this Nphi"); return -1; }
 	s->nlat = nl; s->nlat_2 = nl / 2; s->nphi = np;
 	s->nspat = (unsigned)((long) nl * np);
 	s->nlat_padded = nl;

@@ -1,0 +1,95 @@
+"""The generic phi-FFT kernels (sht_fft_gen.cu) against torch.fft, through the
+FFT stage entry points, at sizes where their pass plans change: one radix, the
+primes alone, two to five passes, each register class, the largest sizes, and
+row counts that end inside a tile.  Bar: 1e-13 of the largest value (a pass of
+radix <= 16 adds a few 2^-53; at most eight passes and their twiddle products)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from tests.common import relerr
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [1, 2, 3, 5, 7, 9, 16, 18, 25, 49, 64, 90, 125, 216, 243, 343, 360, 512, 720, 1000, 1024, 1440, 1680, 2187, 2401, 3000,
+         3125, 4050, 4096, 5040, 5832, 6250, 6300, 6400]
+
+
+@pytest.mark.parametrize("layout", ["theta", "phi"])
+@pytest.mark.parametrize("nphi", SIZES)
+def test_generic_fft_matches_torch(nphi, layout):
+    import shtns_b200
+    from shtns_b200 import capi
+    lib = capi.load()
+    dev = torch.device("cuda:0")
+    phi = layout == "phi"
+    mmax = (nphi - 1) // 2 if nphi % 2 else nphi // 3        # up to the last order below Nyquist, or a zero band
+    if nphi > 1100 and nphi not in (2187, 5040):
+        mmax = min(mmax, 150)                                # fewer orders: quicker plans
+    nlat = 2 * ((mmax + 44) // 2)
+    sh = shtns_b200.sht(max(mmax, 2), mmax)
+    sh.set_grid(nlat, nphi, flags=shtns_b200.sht_quick_init | (shtns_b200.SHT_PHI_CONTIGUOUS if phi else shtns_b200.SHT_THETA_CONTIGUOUS),
+                polar_opt=0.0)
+    lib.shtns_b200_set_option(sh._cfg, 3, 1)
+    lib.cushtns_set_streams(sh._cfg, C.c_void_p(torch.cuda.current_stream().cuda_stream), None)
+    g = torch.Generator(device="cpu").manual_seed(nphi)
+    for nrows, nf, pairs in ((nlat, 2, 0), (2, 1, 0), (10, 3, 0), (38, 1, 8), (38, 1, 1)):
+        lib.shtns_b200_set_option(sh._cfg, 1, pairs)
+        shape = (nf, nrows, nphi) if phi else (nf, nphi, nrows)
+        lib.shtns_set_batch(sh._cfg, nf, sh.nlm, nrows * nphi)
+        if sh.nspat > nrows * nphi and nf > 1:
+            continue                                         # fields of a block lie nspat apart: whole grids and single fields only
+        F = torch.randn((nf, mmax + 1, nrows), dtype=torch.complex128, generator=g)
+        F[:, 0] = F[:, 0].real.to(torch.complex128)
+        F = F.to(dev)
+        v = torch.full(shape, float("nan"), dtype=torch.float64, device=dev)
+        lib.shtns_b200_status()
+        lib.shtns_b200_fourier_synth(sh._cfg, 0, C.c_void_p(F.data_ptr()), C.c_void_p(v.data_ptr()), None, None, nrows, sh.lmax)
+        torch.cuda.synchronize()
+        assert lib.shtns_b200_status() == 0, lib.shtns_b200_last_error().decode()
+        assert lib.shtns_b200_get_option(sh._cfg, 6) == 0
+        z = torch.zeros((nf, nphi // 2 + 1, nrows), dtype=torch.complex128, device=dev)
+        z[:, : mmax + 1] = F
+        want = torch.fft.irfft(z, nphi, dim=1, norm="forward")
+        want = want.transpose(1, 2) if phi else want
+        assert relerr(want.cpu().numpy(), v.cpu().numpy()) < 1e-13, (nrows, nf, pairs)
+        w = torch.randn(shape, dtype=torch.float64, generator=g).to(dev)
+        G = torch.full((nf, mmax + 1, nrows), float("nan"), dtype=torch.complex128, device=dev)
+        lib.shtns_b200_fourier_analys(sh._cfg, 0, C.c_void_p(w.data_ptr()), None, None, C.c_void_p(G.data_ptr()), nrows, sh.lmax)
+        torch.cuda.synchronize()
+        assert lib.shtns_b200_status() == 0, lib.shtns_b200_last_error().decode()
+        R = torch.fft.rfft(w.transpose(1, 2) if phi else w, dim=1, norm="forward")[:, : mmax + 1]
+        assert relerr(R.cpu().numpy(), G.cpu().numpy()) < 1e-13, (nrows, nf, pairs)
+    assert lib.shtns_b200_kernel_errors(sh._cfg) == 0
+
+
+def test_generic_fft_wait_limit_reports_and_recovers():
+    """The staged kernels wait for their tensor copies with a time limit.
+    Option 7 makes them expect 16 bytes more than arrive: the wait gives up
+    after about a second, the flag is set, and the next call is right."""
+    import shtns_b200
+    from shtns_b200 import capi
+    lib = capi.load()
+    dev = torch.device("cuda:0")
+    sh = shtns_b200.sht(40)
+    sh.set_grid(64, 100, flags=shtns_b200.sht_quick_init | shtns_b200.SHT_THETA_CONTIGUOUS, polar_opt=0.0)
+    q = torch.randn(300, sh.nlm, dtype=torch.complex128, device=dev)
+    q.imag[:, :41] = 0
+    v = sh.synth(q)
+    assert lib.shtns_b200_kernel_errors(sh._cfg) == 0
+    assert lib.shtns_b200_set_option(sh._cfg, 7, 16) == 0
+    sh.analys(v[:2])
+    torch.cuda.synchronize()
+    assert lib.shtns_b200_set_option(sh._cfg, 7, 0) == 0
+    lib.shtns_b200_kernel_errors(sh._cfg)                    # small grids may read directly: 0 or 1
+    sh2 = shtns_b200.sht(40)
+    sh2.set_grid(64, 100, flags=shtns_b200.sht_quick_init | shtns_b200.SHT_THETA_CONTIGUOUS, polar_opt=0.0)
+    lib.shtns_b200_set_option(sh2._cfg, 7, 16)
+    sh2.analys(v)
+    assert lib.shtns_b200_kernel_errors(sh2._cfg) == 1
+    assert lib.shtns_b200_kernel_errors(sh2._cfg) == 0
+    back = sh.analys(v)
+    assert lib.shtns_b200_kernel_errors(sh._cfg) == 0
+    assert relerr(q.cpu().numpy(), back.cpu().numpy()) < 1e-12
