@@ -49,16 +49,29 @@ using namespace shtb_fft_grid;
 // 16-byte latitude pairs in global memory).
 template <int... Rs> struct RadixList {};
 
+// Pass chain of nphi = N and complex values per thread D (the CTA has S N / D
+// threads).  Few long passes win where the tile arrives by tensor copies and
+// the shared memory allows two CTAs per SM whatever their threads: each pass is
+// a round trip through shared memory and two barriers.  Measured (FFT stages,
+// synthesis / analysis, us; before: 8 8 8 3, 8 8 4 3, 8 8 4 4 3 and 8 4 4 3 with
+// 8 values per thread): nphi 1536, 96 grids of 768 latitudes 430/399 -> 398/364;
+// 768, 256 x 384 278/243 -> 254/225; 3072, 6 phi-contiguous x 1536 129/140 ->
+// 106/115; 384, 64 phi-contiguous x 192 25.1/26.5 -> 22.5/23.6.  1536 as 12 16 8
+// (12 values per thread) spills: 492/395.  192 as 16 12 or 8 4 6, and two passes
+// for the 96 and 128 of the four-step kernels, were not faster.
 template <int N> struct NphiPlan;
-template <> struct NphiPlan<192>  { using L = RadixList<8, 8, 3>; };
-template <> struct NphiPlan<384>  { using L = RadixList<8, 4, 4, 3>; };
-template <> struct NphiPlan<768>  { using L = RadixList<8, 8, 4, 3>; };
-template <> struct NphiPlan<1536> { using L = RadixList<8, 8, 8, 3>; };
-template <> struct NphiPlan<3072> { using L = RadixList<8, 8, 4, 4, 3>; };
-template <> struct NphiPlan<6144> { using L = RadixList<8, 8, 8, 4, 3>; };
-template <> struct NphiPlan<12288> { using L = RadixList<8, 8, 8, 8, 3>; };
-template <> struct NphiPlan<96>  { using L = RadixList<8, 4, 3>; };
-template <> struct NphiPlan<128> { using L = RadixList<8, 4, 4>; };
+template <> struct NphiPlan<192>  { using L = RadixList<8, 8, 3>; static constexpr int D = 8; };
+template <> struct NphiPlan<384>  { using L = RadixList<8, 8, 6>; static constexpr int D = 8; };
+template <> struct NphiPlan<768>  { using L = RadixList<16, 8, 6>; static constexpr int D = 16; };
+template <> struct NphiPlan<1536> { using L = RadixList<16, 16, 6>; static constexpr int D = 16; };
+template <> struct NphiPlan<3072> { using L = RadixList<16, 16, 12>; static constexpr int D = 16; };
+template <> struct NphiPlan<96>  { using L = RadixList<8, 4, 3>; static constexpr int D = 8; };
+template <> struct NphiPlan<128> { using L = RadixList<8, 4, 4>; static constexpr int D = 8; };
+template <> struct NphiPlan<6144> { using L = RadixList<8, 8, 8, 4, 3>; static constexpr int D = 8; };
+template <> struct NphiPlan<12288> { using L = RadixList<8, 8, 8, 8, 3>; static constexpr int D = 8; };
+
+// CTAs per SM of the prefetching kernels that the shared memory allows
+constexpr int fft4_minb(int SN) { return 6144 / SN < 1 ? 1 : (6144 / SN > 16 ? 16 : 6144 / SN); }
 
 template <int N, int S>
 struct Geo {
@@ -67,8 +80,9 @@ struct Geo {
 	// that the 8 lanes of a 16-byte access phase, on consecutive sequences,
 	// hit distinct banks
 	static constexpr int SEQ = A + (((S >= 8 ? 1 : 8 / S) - A) & 7);
-	// one radix-8 butterfly per thread, at most 768 threads (two or more per thread beyond)
-	static constexpr int T = (S * N / 8 <= 768) ? S * N / 8 : 768;
+	// D values per thread, at most 768 threads (more values per thread beyond)
+	static constexpr int D = NphiPlan<N>::D;
+	static constexpr int T = (S * N / D <= 768) ? S * N / D : 768;
 	static __device__ __forceinline__ int at(int s, int i) { return s * SEQ + i + (i >> 3); }
 };
 
@@ -78,11 +92,14 @@ __device__ __forceinline__ void twiddle(double2* u, const double2* __restrict__ 
 {
 	double2 w1 = __ldg(tw + idx);
 	if (sign < 0) w1.y = -w1.y;
-	double2 w = w1;
-	#pragma unroll
-	for (int q = 1; q < R; q++) {
-		u[q] = cmul(u[q], w);
-		if (q + 1 < R) w = cmul(w, w1);
+	if constexpr (R > 8) twiddles<R>(u, w1);
+	else {
+		double2 w = w1;
+		#pragma unroll
+		for (int q = 1; q < R; q++) {
+			u[q] = cmul(u[q], w);
+			if (q + 1 < R) w = cmul(w, w1);
+		}
 	}
 }
 
@@ -120,41 +137,45 @@ __device__ __forceinline__ void mid_pass(double2* X, const double2* __restrict__
 	__syncthreads();
 }
 
-// Last pass of an analysis chain ending in radix 3 (P = N/3): thread item
-// (s, b), b = 0 .. P/2, runs the butterflies b and P - b of sequence s, which
-// hold both members of the pairs (z_k, z_{N-k}) for k = b, P - b and P + b
-// (b = 0: k = 0, P; b = P/2: k = P/2), and hands each pair to st(s, k, z_k,
-// z_{N-k}).  Every k < N/2 is handed over once; no shared-memory output.
-template <int N, int S, class Store>
+// Last pass of an analysis chain, radix R (P = N/R): thread item (s, b), b = 0
+// .. P/2, runs the butterflies b and P - b of sequence s.  They hold both
+// members of the pairs (z_k, z_{N-k}) for k = b + q P and k = P - b + q P (b =
+// 0 and b = P/2 pair with themselves), and each pair with k < N/2 goes to
+// st(s, k, z_k, z_{N-k}).  Every k < N/2 is handed over once; no shared-memory
+// output.
+template <int N, int S, int R, class Store>
 __device__ __forceinline__ void last_pass_pairs(const double2* X, const double2* __restrict__ tw, int sign, Store& st, int tid)
 {
 	using G = Geo<N, S>;
-	constexpr int P = N / 3, H = P / 2, ITEMS = S * (H + 1), NB = (ITEMS + G::T - 1) / G::T;
+	constexpr int P = N / R, H = P / 2, ITEMS = S * (H + 1), NB = (ITEMS + G::T - 1) / G::T;
+	static_assert(P % 2 == 0, "the pairs of a last pass");
 	#pragma unroll
 	for (int i = 0; i < NB; i++) {
 		const int g = tid + i * G::T;
 		if (g < ITEMS) {
 			const int s = g % S, b = g / S;
-			double2 u[3];
+			double2 u[R];
 			#pragma unroll
-			for (int q = 0; q < 3; q++) u[q] = X[G::at(s, b + q * P)];
-			if (b) twiddle<3>(u, tw, b, sign);
-			Dft<3>::run(u, sign);                       // z_{b + q P} = u[q]
+			for (int q = 0; q < R; q++) u[q] = X[G::at(s, b + q * P)];
+			if (b) twiddle<R>(u, tw, b, sign);
+			Dft<R>::run(u, sign);                       // z_{b + q P} = u[q]
 			if (b == 0) {
-				st(s, 0, u[0], u[0]);
-				st(s, P, u[1], u[2]);
+				#pragma unroll
+				for (int q = 0; 2 * q < R; q++) st(s, q * P, u[q], u[(R - q) % R]);
 			} else if (b == H) {
-				st(s, H, u[0], u[2]);
+				#pragma unroll
+				for (int q = 0; 2 * q + 1 < R; q++) st(s, H + q * P, u[q], u[R - 1 - q]);
 			} else {
 				const int bp = P - b;
-				double2 v[3];
+				double2 v[R];
 				#pragma unroll
-				for (int q = 0; q < 3; q++) v[q] = X[G::at(s, bp + q * P)];
-				twiddle<3>(v, tw, bp, sign);
-				Dft<3>::run(v, sign);                   // z_{P - b + q P} = v[q]
-				st(s, b, u[0], v[2]);
-				st(s, bp, v[0], u[2]);
-				st(s, P + b, u[1], v[1]);
+				for (int q = 0; q < R; q++) v[q] = X[G::at(s, bp + q * P)];
+				twiddle<R>(v, tw, bp, sign);
+				Dft<R>::run(v, sign);                   // z_{P - b + q P} = v[q]
+				#pragma unroll
+				for (int q = 0; 2 * q < R; q++) st(s, b + q * P, u[q], v[R - 1 - q]);
+				#pragma unroll
+				for (int q = 0; 2 * q + 1 < R; q++) st(s, bp + q * P, v[q], u[R - 1 - q]);
 			}
 		}
 	}
@@ -163,7 +184,7 @@ __device__ __forceinline__ void last_pass_pairs(const double2* X, const double2*
 // Pass chain: first pass from a loader, middle passes in shared memory, last
 // pass to shared memory (MODE 0), to a storer (MODE 1), to shared memory in
 // rows of S complex values (MODE 2), or as (z_k, z_{N-k}) pairs to a storer
-// (MODE 3, last radix 3).
+// (MODE 3).
 template <int N, int S, int P, int MODE, int R, int... Rest>
 struct Chain {
 	template <class Store>
@@ -171,8 +192,7 @@ struct Chain {
 	{
 		if constexpr (sizeof...(Rest) == 0) {
 			if constexpr (MODE == 3) {
-				static_assert(R == 3 && P * 3 == N, "the pair pass is the last radix-3 pass");
-				last_pass_pairs<N, S>(X, tw, sign, st, tid);
+				last_pass_pairs<N, S, R>(X, tw, sign, st, tid);
 			} else if constexpr (MODE == 1) {
 				// last pass: k = b (b < P = N/R), outputs b + q*P go to global memory
 				using G = Geo<N, S>;
@@ -525,7 +545,7 @@ __device__ __forceinline__ void store_tile(const CUtensorMap* map, const char* X
 // TOUT: theta-contiguous output written by tensor stores of whole tiles
 // (rows of 2 S latitudes) from X, instead of 16-byte stores per latitude pair
 template <int N, int S, bool TOUT, class G>
-__global__ void __launch_bounds__(Geo<N, S>::T, 768 / Geo<N, S>::T) fft4_synth_kernel(
+__global__ void __launch_bounds__(Geo<N, S>::T, fft4_minb(S * N)) fft4_synth_kernel(
 	const __grid_constant__ CUtensorMap fmap, const __grid_constant__ CUtensorMap o0, const __grid_constant__ CUtensorMap o1,
 	const __grid_constant__ CUtensorMap o2, FftParams p, TmaTiles tt)
 {
@@ -600,7 +620,7 @@ __global__ void __launch_bounds__(Geo<N, S>::T, 768 / Geo<N, S>::T) fft4_synth_k
 }
 
 template <int N, int S, class G>
-__global__ void __launch_bounds__(Geo<N, S>::T, 768 / Geo<N, S>::T) fft4_analys_kernel(
+__global__ void __launch_bounds__(Geo<N, S>::T, fft4_minb(S * N)) fft4_analys_kernel(
 	const __grid_constant__ CUtensorMap m0, const __grid_constant__ CUtensorMap m1, const __grid_constant__ CUtensorMap m2,
 	FftParams p, TmaTiles tt)
 {

@@ -47,3 +47,25 @@ def test_fourier_rows_from_pairs_match_numpy(N):
         a = 0.5 / N * complex(zk.real + wk.real, zk.imag - wk.imag)
         b = 0.5 / N * complex(zk.imag + wk.imag, -(zk.real - wk.real))
         assert abs(a - fa[k]) < 1e-12 and abs(b - fb[k]) < 1e-12
+
+
+@pytest.mark.parametrize("N,R", [(192, 3), (384, 6), (768, 6), (1536, 6), (3072, 12), (24, 2), (64, 8), (40, 5)])
+def test_pairs_of_any_last_radix(N, R):
+    """The same for a last pass of radix R, P = N / R even: butterflies b and
+    P - b hold z_{b + q P} and z_{P - b + q P}, and the partner of k = b + q P is
+    entry R - 1 - q of the other one (b = 0: entry (R - q) mod R of itself)."""
+    P, H = N // R, N // R // 2
+    out = []
+    for b in range(H + 1):
+        u = [b + q * P for q in range(R)]
+        v = [P - b + q * P for q in range(R)]
+        if b == 0:
+            out += [(q * P, u[q], u[(R - q) % R]) for q in range(R) if 2 * q < R]
+        elif b == H:
+            out += [(H + q * P, u[q], u[R - 1 - q]) for q in range(R) if 2 * q + 1 < R]
+        else:
+            out += [(b + q * P, u[q], v[R - 1 - q]) for q in range(R) if 2 * q < R]
+            out += [(P - b + q * P, v[q], u[R - 1 - q]) for q in range(R) if 2 * q + 1 < R]
+    assert sorted(k for k, _, _ in out) == list(range((N + 1) // 2))
+    for k, i, j in out:
+        assert i == k and j == (N - k) % N
