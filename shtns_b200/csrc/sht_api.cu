@@ -185,16 +185,19 @@ void run_analys(shtns_cfg s, int ncomp, const int* types, const double* i0, cons
 	fp.spat_in[0] = i0; fp.spat_in[1] = i1; fp.spat_in[2] = i2;
 	fp.vec2 = aligned16(i0, i1, i2, s->spat_dist);
 	if (s->d_tw4 && !s->phi_contiguous && fp.vec2 && s->fft_generic == 0) {
-		// the four-step FFT analysis of nphi = 12288 needs a grid per field-component of scratch
-		// (without room for it the direct kernels run instead)
+		// the four-step FFT analysis needs a grid per field-component of scratch
+		// (without room for it, or where a stream capture forbids the allocation,
+		// the direct kernels run instead)
 		const size_t b = sizeof(double) * (size_t) j.nfc * s->nphi * s->nlat;
-		if (s->fscr_cap < b) {
+		cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+		const bool grow = s->fscr_cap < b && cudaStreamIsCapturing(s->comp_stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+		if (grow) {
 			if (s->d_fscr) cudaFree(s->d_fscr);
 			s->d_fscr = nullptr; s->fscr_cap = 0;
 			if (cudaMalloc(reinterpret_cast<void**>(&s->d_fscr), b) == cudaSuccess) s->fscr_cap = b;
 			else { cudaGetLastError(); s->d_fscr = nullptr; }
 		}
-		fp.scratch = s->d_fscr;
+		fp.scratch = s->fscr_cap >= b ? s->d_fscr : nullptr;
 	}
 	shtb_stage_begin(s, 3);
 	launch_fft_analys(fp, j.nfc, s->comp_stream);

@@ -65,6 +65,8 @@ template <> struct NphiPlan<384>  { using L = RadixList<8, 8, 6>; static constex
 template <> struct NphiPlan<768>  { using L = RadixList<16, 8, 6>; static constexpr int D = 16; };
 template <> struct NphiPlan<1536> { using L = RadixList<16, 16, 6>; static constexpr int D = 16; };
 template <> struct NphiPlan<3072> { using L = RadixList<16, 16, 12>; static constexpr int D = 16; };
+template <> struct NphiPlan<48>  { using L = RadixList<8, 6>; static constexpr int D = 8; };
+template <> struct NphiPlan<64>  { using L = RadixList<8, 8>; static constexpr int D = 8; };
 template <> struct NphiPlan<96>  { using L = RadixList<8, 4, 3>; static constexpr int D = 8; };
 template <> struct NphiPlan<128> { using L = RadixList<8, 4, 4>; static constexpr int D = 8; };
 template <> struct NphiPlan<6144> { using L = RadixList<8, 8, 8, 4, 3>; static constexpr int D = 8; };
@@ -324,7 +326,8 @@ __global__ void __launch_bounds__(Geo<N, S>::T) fft3_analys_kernel(FftParams p)
 }
 
 // ---------------------------------------------------------------------------
-// Four-step FFT for nphi = N1 N2 = 96 x 128 = 12288 (theta-contiguous grids).
+// Four-step FFT for nphi = N1 N2 = 96 x 128 = 12288 and 64 x 96 = 6144
+// (theta-contiguous grids).
 // With j = j1 + N1 j2 and k = k2 + N2 k1,
 //   exp(s 2 pi i j k / N) = w_N^(j1 k2) w_N1^(j1 k1) w_N2^(j2 k2),
 // so a length-N transform is N2 transforms of length N1 (over k1), a twiddle
@@ -813,7 +816,10 @@ bool launch_fft4_n(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 }
 
 // four-step path on theta-contiguous grids with 16-byte aligned latitude pairs
-// and (analysis) a scratch grid; false otherwise.
+// and (analysis) a scratch grid; false otherwise.  Against the one-pass kernels,
+// synthesis / analysis: nphi 6144, 8 grids of 3072 latitudes 1552/1155 ->
+// 866/803 us; the synthesis of nphi 3072, 32 grids of 1536 latitudes 1417 -> 783
+// us (its one-pass kernel stores 16 bytes of each grid row, half a sector).
 template <int N1, int N2>
 bool launch_fourstep(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 {
@@ -845,7 +851,11 @@ void set_fourstep_limits()
 
 bool launch_fused(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 {
-	if (launch_fourstep<96, 128>(p, nfc, st, synth)) return true;
+	if (launch_fourstep<96, 128>(p, nfc, st, synth) || launch_fourstep<64, 96>(p, nfc, st, synth)) return true;
+	// nphi 3072: the synthesis of grids that do not stay in the L2 cache, where
+	// the half sectors of the one-pass kernel would be completed (3 grids of 1536
+	// latitudes: 100 -> 83 us)
+	if (synth && (size_t) nfc * p.N * p.nlat * 8 > ((size_t) 96 << 20) && launch_fourstep<48, 64>(p, nfc, st, synth)) return true;
 	if (p.generic == 0 || p.generic == 3) {
 		bool done = false;
 		switch (p.N) {
@@ -960,12 +970,15 @@ void launch_fft_analys(const FftParams& p, int nfc, cudaStream_t st)
 bool fft_fourstep_factors(int N, int& n1, int& n2)
 {
 	if (N == 12288) { n1 = 96; n2 = 128; return true; }
+	if (N == 6144) { n1 = 64; n2 = 96; return true; }
+	if (N == 3072) { n1 = 48; n2 = 64; return true; }
 	return false;
 }
 
 void fft_set_smem_limits()
 {
 	set_fourstep_limits<96, 128>();
+	set_fourstep_limits<64, 96>();
 	tensor_map_encoder();    // resolved here, outside any stream capture
 	sm_count();
 	set_fused_limits<192>(); set_fused_limits<384>(); set_fused_limits<768>();
