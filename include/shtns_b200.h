@@ -71,6 +71,9 @@ int shtns_b200_polar_rows(shtns_cfg, int* tm);
  * No counterpart in SHTns 3.5.2. */
 void cu_SH_to_spat_adjoint(shtns_cfg, double *Vg, cplx *Qg, int ltr);
 void cu_spat_to_SH_adjoint(shtns_cfg, cplx *Qg, double *Vg, int ltr);
+/* The same with FP32 arrays (computed in FP64, as the _float transforms). */
+void cu_SH_to_spat_adjoint_float(shtns_cfg, float *Vg, cplx_f *Qg, int ltr);
+void cu_spat_to_SH_adjoint_float(shtns_cfg, cplx_f *Qg, float *Vg, int ltr);
 
 /* Tuning options of a plan.  option 1: latitude pairs per FFT CTA (1, 2, 4,
  * 8 where the fused chain's buffer fits; 0 = automatic); option 2: recurrence checkpoint spacing (8, 16, 32; rebuilds

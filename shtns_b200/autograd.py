@@ -10,7 +10,7 @@ complex coefficients follow PyTorch's convention dL/dRe + i dL/dIm, so the
 real-valued transforms and their adjoints are exact transposes.
 
 Inputs may be complex128/float64 (FP64) or complex64/float32 (FP32: computed
-in FP64 on the device and rounded back to FP32).  Leading dimensions batch.
+in FP64 by kernels that read and write the FP32 arrays).  Leading dimensions batch.
 """
 import ctypes as C
 
@@ -27,58 +27,49 @@ def _call(sh, fn, src, nfields, dst, ltr):
     capi.check(lib)
 
 
-def _spec64(q):
-    return q.to(torch.complex128).contiguous()
+def _to_spat(sh, fn, q, out, ltr):
+    """fn (synthesis or adjoint of the analysis) of coefficients q into a grid
+    of type out.  FP32 arrays go to the FP32 entry points as they are; any
+    other pair of types is converted to FP64 and back."""
+    single = q.dtype == torch.complex64 and out == torch.float32
+    q = (q if single else q.to(torch.complex128)).contiguous().resolve_conj().resolve_neg()
+    nf = q.numel() // sh.nlm
+    v = torch.empty(tuple(q.shape[:-1]) + sh.spat_shape, dtype=torch.float32 if single else torch.float64, device=q.device)
+    _call(sh, fn + "_float" if single else fn, q, nf, v, ltr)
+    return v.to(out)
 
 
-def _spat64(v):
-    return v.to(torch.float64).contiguous()
+def _to_spec(sh, fn, v, out, ltr):
+    """fn (analysis or adjoint of the synthesis) of a grid v into coefficients
+    of type out (types as in _to_spat)."""
+    single = v.dtype == torch.float32 and out == torch.complex64
+    v = (v if single else v.to(torch.float64)).contiguous().resolve_neg()
+    nf = v.numel() // sh.nspat
+    q = torch.empty(tuple(v.shape[:-2]) + (sh.nlm,), dtype=torch.complex64 if single else torch.complex128, device=v.device)
+    _call(sh, fn + "_float" if single else fn, v, nf, q, ltr)
+    return q.to(out)
 
 
 class _Synth(torch.autograd.Function):
     @staticmethod
     def forward(ctx, sh, q, ltr):
-        ctx.sh, ctx.ltr = sh, ltr
-        ctx.in_dtype = q.dtype
-        q64 = _spec64(q)
-        lead = tuple(q64.shape[:-1])
-        nf = q64.numel() // sh.nlm
-        v = torch.empty(lead + sh.spat_shape, dtype=torch.float64, device=q.device)
-        _call(sh, "cu_SH_to_spat", q64, nf, v, ltr)
-        return v if q.dtype == torch.complex128 else v.to(torch.float32)
+        ctx.sh, ctx.ltr, ctx.in_dtype = sh, ltr, q.dtype
+        return _to_spat(sh, "cu_SH_to_spat", q, torch.float64 if q.dtype == torch.complex128 else torch.float32, ltr)
 
     @staticmethod
     def backward(ctx, g):
-        sh = ctx.sh
-        g64 = _spat64(g)
-        lead = tuple(g64.shape[:-2])
-        nf = g64.numel() // sh.nspat
-        qg = torch.empty(lead + (sh.nlm,), dtype=torch.complex128, device=g.device)
-        _call(sh, "cu_SH_to_spat_adjoint", g64, nf, qg, ctx.ltr)
-        return None, qg.to(ctx.in_dtype), None
+        return None, _to_spec(ctx.sh, "cu_SH_to_spat_adjoint", g, ctx.in_dtype, ctx.ltr), None
 
 
 class _Analys(torch.autograd.Function):
     @staticmethod
     def forward(ctx, sh, v, ltr):
-        ctx.sh, ctx.ltr = sh, ltr
-        ctx.in_dtype = v.dtype
-        v64 = _spat64(v)
-        lead = tuple(v64.shape[:-2])
-        nf = v64.numel() // sh.nspat
-        q = torch.empty(lead + (sh.nlm,), dtype=torch.complex128, device=v.device)
-        _call(sh, "cu_spat_to_SH", v64, nf, q, ltr)
-        return q if v.dtype == torch.float64 else q.to(torch.complex64)
+        ctx.sh, ctx.ltr, ctx.in_dtype = sh, ltr, v.dtype
+        return _to_spec(sh, "cu_spat_to_SH", v, torch.complex128 if v.dtype == torch.float64 else torch.complex64, ltr)
 
     @staticmethod
     def backward(ctx, h):
-        sh = ctx.sh
-        h64 = _spec64(h)
-        lead = tuple(h64.shape[:-1])
-        nf = h64.numel() // sh.nlm
-        vg = torch.empty(lead + sh.spat_shape, dtype=torch.float64, device=h.device)
-        _call(sh, "cu_spat_to_SH_adjoint", h64, nf, vg, ctx.ltr)
-        return None, vg.to(ctx.in_dtype), None
+        return None, _to_spat(ctx.sh, "cu_spat_to_SH_adjoint", h, ctx.in_dtype, ctx.ltr), None
 
 
 def synth(sh, q, ltr=None):

@@ -116,6 +116,8 @@ PROTOTYPES = {
     "cu_SH_to_spat_noalloc": (None, [CFG, P, P, I]),
     "cu_SH_to_spat_adjoint": (None, [CFG, P, P, I]),
     "cu_spat_to_SH_adjoint": (None, [CFG, P, P, I]),
+    "cu_SH_to_spat_adjoint_float": (None, [CFG, P, P, I]),
+    "cu_spat_to_SH_adjoint_float": (None, [CFG, P, P, I]),
     "shtns_b200_set_option": (I, [CFG, I, I]),
     "SH_to_spat_cplx": (None, [CFG, P, P]),
     "spat_cplx_to_SH": (None, [CFG, P, P]),

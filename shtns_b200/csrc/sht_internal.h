@@ -216,6 +216,7 @@ struct PrepParams {
 	int neg_from;                        // > 0: fields f >= neg_from use -m in the vector terms (complex-field transforms)
 	const double2 *Q, *S, *T;            // spectral inputs (may be null: zeros)
 	double2 *Qo, *So, *To;               // spectral outputs (analysis)
+	int f32;                             // the spectral arrays are float2 (the pointers above point to float2)
 	long spec_dist;
 	const double *xs, *xa, *stdt_lo, *stdt_hi, *van_lo, *van_hi, *l2;
 	MTables mt;

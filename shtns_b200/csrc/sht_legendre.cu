@@ -100,7 +100,8 @@ __global__ void ck_kernel(int nlat_2, int mres, int seg, const double* __restric
 // scalar fields at lmax 4095: 684 instead of 452).
 __host__ __device__ constexpr int pt_items(int PF) { return PF <= 2 ? 256 : 512; }     // (row, field-component) items of a CTA
 
-template <int PF>
+// C: coefficient type, double2, or float2 for the single-precision transforms.
+template <int PF, class C>
 __global__ void __launch_bounds__(256, 6) prep_synth_kernel(PrepParams p)
 {
 	constexpr int PT_F = PF, PT_K = pt_items(PF) / PF;
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(256, 6) prep_synth_kernel(PrepParams p)
 	const int q0 = (WP == 1) ? warp : warp / WP, i0 = lane + 32 * (warp % WP);
 	#pragma unroll
 	for (int h = 0; h < PW; h += QB) {
-		const double2* base[QB];
+		const C* base[QB];
 		#pragma unroll
 		for (int qi = 0; qi < QB; qi++) {
 			const int q = q0 + 8 * (h + qi), a = q / PT_F, fc = fc0 + q % PT_F;
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(256, 6) prep_synth_kernel(PrepParams p)
 			if (fc < nfc && (a == 0 || vec)) {
 				const int comp = fc / p.nf, f = fc - comp * p.nf;
 				const double2* x = (p.comp_type[comp] == 0) ? (a == 0 ? p.Q : nullptr) : (a == 0 ? p.S : p.T);
-				if (x) base[qi] = x + off + (long)f * p.spec_dist + d0;
+				if (x) base[qi] = reinterpret_cast<const C*>(x) + off + (long)f * p.spec_dist + d0;
 			}
 		}
 		#pragma unroll
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(256, 6) prep_synth_kernel(PrepParams p)
 					const int i = i0 + 32 * WP * (u0 + u), d = d0 + i;
 					v[qi][u] = make_double2(0.0, 0.0);
 					if (u0 + u < NI && base[qi] && i < PT_W && d >= 0 && d <= lrel_max) {
-						const double2 x = base[qi][i];
+						const C x = base[qi][i];
 						v[qi][u] = make_double2(x.x, m0 ? 0.0 : x.y);
 					}
 				}
@@ -268,7 +269,7 @@ __device__ __forceinline__ double2 ish_inv_s(const double2 (*E)[PE_S], const dou
 	return make_double2(x2 * o.x, x2 * o.y);
 }
 
-template <int PF>
+template <int PF, class C>
 __global__ void __launch_bounds__(256) post_analys_kernel(PrepParams p)
 {
 	constexpr int PE_F = PF, PE_J = PostTile<PF>::J, PE_R = PostTile<PF>::R, PE_S = PostTile<PF>::S;
@@ -345,6 +346,11 @@ __global__ void __launch_bounds__(256) post_analys_kernel(PrepParams p)
 	__syncthreads();
 	const double em = (p.msign < 0) ? -(double) m : (double) m;   // signed m (negative orders of the _ml transforms)
 	const int lane = threadIdx.x & 31;
+	auto store = [&](double2* to, long at, double2 v) {
+		C x;
+		x.x = v.x; x.y = v.y;
+		reinterpret_cast<C*>(to)[at] = x;
+	};
 	// a warp covers 32 consecutive degrees of one field: each lane forms its
 	// own degree in the spectral basis and takes the neighbours (j -/+ 1) of
 	// the vector formulas from the adjacent lanes
@@ -362,7 +368,7 @@ __global__ void __launch_bounds__(256) post_analys_kernel(PrepParams p)
 				q = ish_inv_s(sv, xs, kb, fl, j);
 				if (m == 0) q.y = 0.0;
 			}
-			p.Qo[o] = q;
+			store(p.Qo, o, q);
 			continue;
 		}
 		const bool fv = !zero_m && f < p.nf && j < nl + 1;   // rows staged: degrees up to nl
@@ -388,8 +394,8 @@ __global__ void __launch_bounds__(256) post_analys_kernel(PrepParams p)
 			t = make_double2(-(-emf * v0.y - mxw_r) * l2, -(emf * v0.x - mxw_i) * l2);
 			if (m == 0) { s.y = 0.0; t.y = 0.0; }
 		}
-		p.So[o] = s;
-		p.To[o] = t;
+		store(p.So, o, s);
+		store(p.To, o, t);
 	}
 }
 
@@ -466,13 +472,18 @@ void launch_prep_synth(const PrepParams& p, cudaStream_t st)
 		dim3 grid((kmax0 + K - 1) / K, (nfc + PF - 1) / PF, p.mlim + 1 - p.im0);
 		kern<<<grid, 256, 0, st>>>(p);
 	};
-	switch (tile_fields(nfc)) {
-		case 1: go(prep_synth_kernel<1>, 1); break;
-		case 2: go(prep_synth_kernel<2>, 2); break;
-		case 4: go(prep_synth_kernel<4>, 4); break;
-		case 8: go(prep_synth_kernel<8>, 8); break;
-		default: go(prep_synth_kernel<16>, 16); break;
-	}
+	auto pick = [&](auto c) {
+		using C = decltype(c);
+		switch (tile_fields(nfc)) {
+			case 1: go(prep_synth_kernel<1, C>, 1); break;
+			case 2: go(prep_synth_kernel<2, C>, 2); break;
+			case 4: go(prep_synth_kernel<4, C>, 4); break;
+			case 8: go(prep_synth_kernel<8, C>, 8); break;
+			default: go(prep_synth_kernel<16, C>, 16); break;
+		}
+	};
+	if (p.f32) pick(float2{});
+	else pick(double2{});
 	shtb_count_launch();
 }
 
@@ -578,12 +589,17 @@ void launch_post_analys_m(const PrepParams& p, int mmax, cudaStream_t st)
 		dim3 grid((p.lmax + J) / J, (p.nf + PF - 1) / PF * ngroups, mmax + 1 - p.im0);
 		kern<<<grid, 256, 0, st>>>(p);
 	};
-	switch (tile_fields(p.nf)) {
-		case 1: go(post_analys_kernel<1>, 1, PostTile<1>::J); break;
-		case 2: case 4: go(post_analys_kernel<4>, 4, PostTile<4>::J); break;
-		case 8: go(post_analys_kernel<8>, 8, PostTile<8>::J); break;
-		default: go(post_analys_kernel<16>, 16, PostTile<16>::J); break;
-	}
+	auto pick = [&](auto c) {
+		using C = decltype(c);
+		switch (tile_fields(p.nf)) {
+			case 1: go(post_analys_kernel<1, C>, 1, PostTile<1>::J); break;
+			case 2: case 4: go(post_analys_kernel<4, C>, 4, PostTile<4>::J); break;
+			case 8: go(post_analys_kernel<8, C>, 8, PostTile<8>::J); break;
+			default: go(post_analys_kernel<16, C>, 16, PostTile<16>::J); break;
+		}
+	};
+	if (p.f32) pick(float2{});
+	else pick(double2{});
 	shtb_count_launch();
 }
 
