@@ -75,6 +75,15 @@ void cu_spat_to_SH_adjoint(shtns_cfg, cplx *Qg, double *Vg, int ltr);
 void cu_SH_to_spat_adjoint_float(shtns_cfg, float *Vg, cplx_f *Qg, int ltr);
 void cu_spat_to_SH_adjoint_float(shtns_cfg, cplx_f *Qg, float *Vg, int ltr);
 
+/* shtns_set_batch (dense fields), cushtns_set_streams and one device transform
+ * in one call, for bindings whose cost per call counts.  kind: 0 SH_to_spat,
+ * 1 SHsphtor_to_spat, 2 SHqst_to_spat, 3 spat_to_SH, 4 spat_to_SHsphtor,
+ * 5 spat_to_SHqst, 6 SH_to_spat_adjoint, 7 spat_to_SH_adjoint, and 8 to 11 the
+ * _float forms of 0, 3, 6, 7; a .. f are the arrays in the order of the cu_*
+ * function, the rest null.  Returns shtns_b200_status(). */
+int shtns_b200_transform(shtns_cfg, cudaStream_t stream, int howmany, int kind, void *a, void *b, void *c, void *d,
+                         void *e, void *f, int ltr);
+
 /* Tuning options of a plan.  option 1: latitude pairs per FFT CTA (1, 2, 4,
  * 8 where the fused chain's buffer fits; 0 = automatic); option 2: recurrence checkpoint spacing (8, 16, 32; rebuilds
  * the checkpoint table; not for clones or plans that have clones); option 3:

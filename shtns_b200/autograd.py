@@ -12,19 +12,11 @@ real-valued transforms and their adjoints are exact transposes.
 Inputs may be complex128/float64 (FP64) or complex64/float32 (FP32: computed
 in FP64 by kernels that read and write the FP32 arrays).  Leading dimensions batch.
 """
-import ctypes as C
-
 import torch
 
-from . import capi
 
-
-def _call(sh, fn, src, nfields, dst, ltr):
-    lib = sh._lib
-    sh._batch(nfields)
-    sh._stream()
-    getattr(lib, fn)(sh._cfg, C.c_void_p(src.data_ptr()), C.c_void_p(dst.data_ptr()), int(ltr))
-    capi.check(lib)
+# kinds of shtns_b200_transform: FP64, and FP32 arrays
+_KIND = {"synth": (0, 8), "analys": (3, 9), "synth_adjoint": (6, 10), "analys_adjoint": (7, 11)}
 
 
 def _to_spat(sh, fn, q, out, ltr):
@@ -35,7 +27,7 @@ def _to_spat(sh, fn, q, out, ltr):
     q = (q if single else q.to(torch.complex128)).contiguous().resolve_conj().resolve_neg()
     nf = q.numel() // sh.nlm
     v = torch.empty(tuple(q.shape[:-1]) + sh.spat_shape, dtype=torch.float32 if single else torch.float64, device=q.device)
-    _call(sh, fn + "_float" if single else fn, q, nf, v, ltr)
+    sh._transform(_KIND[fn][single], nf, [q], [v], ltr)
     return v.to(out)
 
 
@@ -46,7 +38,7 @@ def _to_spec(sh, fn, v, out, ltr):
     v = (v if single else v.to(torch.float64)).contiguous().resolve_neg()
     nf = v.numel() // sh.nspat
     q = torch.empty(tuple(v.shape[:-2]) + (sh.nlm,), dtype=torch.complex64 if single else torch.complex128, device=v.device)
-    _call(sh, fn + "_float" if single else fn, v, nf, q, ltr)
+    sh._transform(_KIND[fn][single], nf, [v], [q], ltr)
     return q.to(out)
 
 
@@ -54,22 +46,22 @@ class _Synth(torch.autograd.Function):
     @staticmethod
     def forward(ctx, sh, q, ltr):
         ctx.sh, ctx.ltr, ctx.in_dtype = sh, ltr, q.dtype
-        return _to_spat(sh, "cu_SH_to_spat", q, torch.float64 if q.dtype == torch.complex128 else torch.float32, ltr)
+        return _to_spat(sh, "synth", q, torch.float64 if q.dtype == torch.complex128 else torch.float32, ltr)
 
     @staticmethod
     def backward(ctx, g):
-        return None, _to_spec(ctx.sh, "cu_SH_to_spat_adjoint", g, ctx.in_dtype, ctx.ltr), None
+        return None, _to_spec(ctx.sh, "synth_adjoint", g, ctx.in_dtype, ctx.ltr), None
 
 
 class _Analys(torch.autograd.Function):
     @staticmethod
     def forward(ctx, sh, v, ltr):
         ctx.sh, ctx.ltr, ctx.in_dtype = sh, ltr, v.dtype
-        return _to_spec(sh, "cu_spat_to_SH", v, torch.complex128 if v.dtype == torch.float64 else torch.complex64, ltr)
+        return _to_spec(sh, "analys", v, torch.complex128 if v.dtype == torch.float64 else torch.complex64, ltr)
 
     @staticmethod
     def backward(ctx, h):
-        return None, _to_spat(ctx.sh, "cu_spat_to_SH_adjoint", h, ctx.in_dtype, ctx.ltr), None
+        return None, _to_spat(ctx.sh, "analys_adjoint", h, ctx.in_dtype, ctx.ltr), None
 
 
 def synth(sh, q, ltr=None):

@@ -118,6 +118,7 @@ PROTOTYPES = {
     "cu_spat_to_SH_adjoint": (None, [CFG, P, P, I]),
     "cu_SH_to_spat_adjoint_float": (None, [CFG, P, P, I]),
     "cu_spat_to_SH_adjoint_float": (None, [CFG, P, P, I]),
+    "shtns_b200_transform": (I, [CFG, P, I, I, P, P, P, P, P, P, I]),
     "shtns_b200_set_option": (I, [CFG, I, I]),
     "SH_to_spat_cplx": (None, [CFG, P, P]),
     "spat_cplx_to_SH": (None, [CFG, P, P]),

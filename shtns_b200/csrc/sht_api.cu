@@ -517,6 +517,35 @@ extern "C" void cu_spat_to_SH_float(shtns_cfg s, float* Vr, cplx_f* Qlm, int ltr
 extern "C" void cu_SH_to_spat_adjoint_float(shtns_cfg s, float* Vg, cplx_f* Qg, int ltr) { analys_float(s, Vg, Qg, ltr, 1); }
 extern "C" void cu_spat_to_SH_adjoint_float(shtns_cfg s, cplx_f* Qg, float* Vg, int ltr) { synth_float(s, Qg, Vg, ltr, 1); }
 
+// One call for a binding (shtns_b200.h): batch, stream, transform and status.
+extern "C" int shtns_b200_transform(shtns_cfg s, cudaStream_t stream, int howmany, int kind, void* a, void* b, void* c,
+                                    void* d, void* e, void* f, int ltr)
+{
+	if (shtns_set_batch(s, howmany, 0, 0) == 0) {
+		cushtns_set_streams(s, stream, nullptr);
+		auto q = [](void* x) { return static_cast<cplx*>(x); };
+		auto v = [](void* x) { return static_cast<double*>(x); };
+		auto qf = [](void* x) { return static_cast<cplx_f*>(x); };
+		auto vf = [](void* x) { return static_cast<float*>(x); };
+		switch (kind) {
+			case 0: cu_SH_to_spat(s, q(a), v(b), ltr); break;
+			case 1: cu_SHsphtor_to_spat(s, q(a), q(b), v(c), v(d), ltr); break;
+			case 2: cu_SHqst_to_spat(s, q(a), q(b), q(c), v(d), v(e), v(f), ltr); break;
+			case 3: cu_spat_to_SH(s, v(a), q(b), ltr); break;
+			case 4: cu_spat_to_SHsphtor(s, v(a), v(b), q(c), q(d), ltr); break;
+			case 5: cu_spat_to_SHqst(s, v(a), v(b), v(c), q(d), q(e), q(f), ltr); break;
+			case 6: cu_SH_to_spat_adjoint(s, v(a), q(b), ltr); break;
+			case 7: cu_spat_to_SH_adjoint(s, q(a), v(b), ltr); break;
+			case 8: cu_SH_to_spat_float(s, qf(a), vf(b), ltr); break;
+			case 9: cu_spat_to_SH_float(s, vf(a), qf(b), ltr); break;
+			case 10: cu_SH_to_spat_adjoint_float(s, vf(a), qf(b), ltr); break;
+			case 11: cu_spat_to_SH_adjoint_float(s, qf(a), vf(b), ltr); break;
+			default: shtb_set_error(1, "shtns_b200_transform: unknown kind");
+		}
+	}
+	return shtns_b200_status();
+}
+
 // ---- host-pointer API (shtns.h) ----
 extern "C" void SH_to_spat(shtns_cfg s, cplx* Qlm, double* Vr) { h_synth(s, 1, T_SCAL, Qlm, nullptr, nullptr, Vr, nullptr, nullptr, s ? s->lmax : 0); }
 extern "C" void SH_to_spat_l(shtns_cfg s, cplx* Qlm, double* Vr, int ltr) { h_synth(s, 1, T_SCAL, Qlm, nullptr, nullptr, Vr, nullptr, nullptr, ltr); }

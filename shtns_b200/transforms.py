@@ -272,7 +272,6 @@ class sht:
                 raise RuntimeError("spectral tensors must be CUDA complex128 with last dimension nlm")
             q.append(a.contiguous())
         lead = tuple(q[0].shape[:-1])
-        nf = int(np.prod(lead)) if lead else 1
         outs = [torch.empty(lead + self.spat_shape, dtype=torch.float64, device=q[0].device) for _ in q]
         self.synth_into(q, outs, ltr)
         return outs[0] if len(outs) == 1 else tuple(outs)
@@ -291,37 +290,21 @@ class sht:
     def synth_into(self, q, outs, ltr=None):
         """Device synthesis into preallocated tensors (no allocation by torch):
         q: list of 1-3 complex128 CUDA tensors (..., nlm); outs: float64 (..., *spat_shape)."""
-        ltr = self.lmax if ltr is None else int(ltr)
-        nf = q[0].numel() // self.nlm
-        self._batch(nf)
-        self._stream()
-        P = [C.c_void_p(x.data_ptr()) for x in q]
-        O = [C.c_void_p(x.data_ptr()) for x in outs]
-        L = self._lib
-        if len(q) == 1:
-            L.cu_SH_to_spat(self._cfg, P[0], O[0], ltr)
-        elif len(q) == 2:
-            L.cu_SHsphtor_to_spat(self._cfg, P[0], P[1], O[0], O[1], ltr)
-        else:
-            L.cu_SHqst_to_spat(self._cfg, P[0], P[1], P[2], O[0], O[1], O[2], ltr)
-        capi.check(L)
+        self._transform(len(q) - 1, q[0].numel() // self.nlm, q, outs, ltr)
 
     def analys_into(self, v, outs, ltr=None):
         """Device analysis into preallocated tensors (see synth_into)."""
-        ltr = self.lmax if ltr is None else int(ltr)
-        nf = v[0].numel() // self.nspat
-        self._batch(nf)
-        self._stream()
-        P = [C.c_void_p(x.data_ptr()) for x in v]
-        O = [C.c_void_p(x.data_ptr()) for x in outs]
-        L = self._lib
-        if len(v) == 1:
-            L.cu_spat_to_SH(self._cfg, P[0], O[0], ltr)
-        elif len(v) == 2:
-            L.cu_spat_to_SHsphtor(self._cfg, P[0], P[1], O[0], O[1], ltr)
-        else:
-            L.cu_spat_to_SHqst(self._cfg, P[0], P[1], P[2], O[0], O[1], O[2], ltr)
-        capi.check(L)
+        self._transform(len(v) + 2, v[0].numel() // self.nspat, v, outs, ltr)
+
+    def _transform(self, kind, nf, src, dst, ltr):
+        """One device transform of nf fields on torch's current stream (kinds
+        of shtns_b200_transform): one foreign call, as its cost counts on small fields."""
+        p = [x.data_ptr() for x in src] + [x.data_ptr() for x in dst]
+        p += [None] * (6 - len(p))
+        lib = self._lib
+        if lib.shtns_b200_transform(self._cfg, torch.cuda.current_stream().cuda_stream, nf, kind, *p,
+                                    self.lmax if ltr is None else int(ltr)):
+            raise SHTError(lib.shtns_b200_last_error().decode())
 
     # ---------------- fixed order, no FFT (shtns_numpy.i:661-704) ----------------
     def _ml_check(self, im, spec, spat):
