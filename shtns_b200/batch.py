@@ -1,9 +1,11 @@
 """Many scalar fields of uneven lmax, each on its own Gauss grid.
 
-`PlanGroup` wraps the plan-group C API (shtns_b200_group_*): the Legendre
-stage of every plan of the group runs as ONE persistent launch whose CTAs take
-(plan, order m, tile) work items from a queue sorted by decreasing cost, and
-every launch of a group transform goes to one stream.
+`PlanGroup` wraps the plan-group C API (shtns_b200_group_*): each plan's
+kernels (prologue, its own Legendre kernels, FFT) run chained on a side stream
+of the group, concurrently with the other plans', forked from and joined to
+one stream.  With group option 5 = 0 the Legendre stage of every plan runs as
+ONE persistent launch instead, whose CTAs take (plan, order m, tile) work items
+from a queue sorted by decreasing cost.
 
 `UnevenBatch` buckets fields by lmax (one plan per distinct lmax, grid
 nlat = 3(lmax+1)/2 rounded up to even, nphi = 2 nlat), keeps the fields of a
@@ -44,7 +46,7 @@ def grid_for(lmax):
 
 
 class PlanGroup:
-    """One persistent Legendre launch over several plans (shtns_b200_group_*).
+    """Transforms of several plans in one call (shtns_b200_group_*).
 
     plans: list of shtns_b200.sht with grids set, on one device.  Transforms
     take per-plan lists of CUDA tensors; a plan with no fields is skipped.
@@ -208,11 +210,11 @@ class UnevenBatch:
 
     # ---------------- transforms ----------------
     def synth(self):
-        """Synthesis of every field (Q -> V): one persistent Legendre launch."""
+        """Synthesis of every field (Q -> V)."""
         self.group.synth_into(self.Q, self.V)
 
     def analys(self):
-        """Analysis of every field (V -> R): one persistent Legendre launch."""
+        """Analysis of every field (V -> R)."""
         self.group.analys_into(self.V, self.R)
 
     def pair(self):
