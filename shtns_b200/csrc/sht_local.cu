@@ -27,6 +27,8 @@
 #include <cstdint>
 #include <cmath>
 #include <vector>
+#include <algorithm>
+#include <type_traits>
 
 namespace {
 
@@ -253,6 +255,240 @@ __global__ void __launch_bounds__(PT_THREADS) point_kernel(LocalParams p, const 
 			o0[pt] = s[0];
 			if (ncomp > 1) { o1[pt] = s[1]; o2[pt] = s[2]; }
 		}
+	}
+}
+
+// ---------------------------------------------------------------------------
+// Values at many points.  A lane owns P points, a warp a set of orders, and the
+// W warps of a CTA share the points: at the end their sums meet in shared
+// memory.  The recurrence constants and coefficients of a degree are the same
+// for every lane, so their loads are broadcasts (the CTA-per-point kernel
+// above has a thread per order: 32 lines per load instruction, and the
+// derivative of every Legendre value, which a scalar field does not need).
+// Bound: the FP64 pipe, 5 instructions per coefficient and point (scalar).
+// Orders are dealt to the warps in a snake; sin^(m-1) goes from one order of a
+// warp to its next by a product with an extended exponent, e^(i m phi) by a
+// rotation that starts anew from sincos every 8 orders.
+// Measured at lmax 255, 65536 points, one scalar field: 14.56 -> 1.14 ms, 9.5
+// TFLOP/s of 33.8 (a CTA per point: see above)
+//
+// Degrees go in blocks of 8.  While some lane of the warp still carries an
+// exponent (E != 0: values below 2^-LOC_FOLD), a block adds only the lanes
+// without one and looks for values that have grown at its end: 8 steps grow by
+// less than 2^60 (a_l < 2^7 up to lmax 8000).  A value above PTS_BIG is folded
+// back if that leaves it above 2^-LOC_FOLD, else scaled down by 2^400, so an
+// exponent that stays is below -LOC_FOLD and the terms left out are below
+// 2^(400 + 60 - LOC_FOLD).
+#define PTS_BIG 0x1p400
+#define PTS_ROT 8
+
+// st^n = y 2^E, y in [0.5, 1) (n = 0: y = 1; st = 0: y = 0)
+__device__ __forceinline__ void pow_ext(double st, int n, double& y, int& E)
+{
+	y = 1.0; E = 0;
+	if (n == 0) return;
+	if (st == 0.0) { y = 0.0; return; }
+	int be, te;
+	double b = frexp(st, &be);
+	for (; n; n >>= 1) {
+		if (n & 1) { y = frexp(y * b, &te); E += be + te; }
+		b = frexp(b * b, &te); be = 2 * be + te;
+	}
+}
+
+// sin and cos of n x with the rounding of the product taken into account
+__device__ __forceinline__ void sincos_mul(double n, double x, double& sn, double& cs)
+{
+	const double p = n * x, e = fma(n, x, -p);
+	double s0, c0;
+	sincos(p, &s0, &c0);
+	sn = fma(e, c0, s0);
+	cs = fma(-e, s0, c0);
+}
+
+template <int NC>
+struct PtsState {
+	double y0, y1, d0, d1;           // Legendre values of degrees l - 1, l, and their derivatives (NC = 3)
+	double2 q, sdt, tdt, sy, ty;
+	int E;
+};
+
+template <int NC, bool GATE>
+__device__ __forceinline__ void pts_add(PtsState<NC>& z, double2 q, double2 s, double2 t)
+{
+	double y = z.y1, d = z.d1;
+	if (GATE && z.E) { y = 0.0; d = 0.0; }
+	z.q = cfma(y, q, z.q);
+	if constexpr (NC == 3) {
+		z.sdt = cfma(d, s, z.sdt); z.sy = cfma(y, s, z.sy);
+		z.tdt = cfma(d, t, z.tdt); z.ty = cfma(y, t, z.ty);
+	}
+}
+
+template <int NC, int P>
+__global__ void __launch_bounds__(512) points_kernel(LocalParams p, const double* __restrict__ cost,
+                                                     const double* __restrict__ phi, int npts, double* o0, double* o1, double* o2)
+{
+	constexpr int NV = (NC == 3) ? 4 : 2;      // (b_l, a_l), Q and, for vectors, S, T
+	extern __shared__ __align__(16) double2 pts_smem[];
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
+	double2 (*stage)[NV] = reinterpret_cast<double2 (*)[NV]>(pts_smem) + 64 * w;      // two chunks of 32 degrees
+	double x[P], st[P], ph[P], v[P][NC], sp[P], stA[P], stB[P], rcA[P], rsA[P], rcB[P], rsB[P], cs[P], sn[P];
+	int spE[P], eA[P], eB[P];
+	// snake: warp w takes order i W + w in even rounds i, i W + W - 1 - w in odd ones
+	const int dA = 2 * (W - w) - 1, dB = 2 * w + 1;      // orders from an even round to the next, and from an odd one
+	#pragma unroll
+	for (int u = 0; u < P; u++) {
+		const int pt = min(blockIdx.x * 32 * P + u * 32 + lane, npts - 1);
+		x[u] = cost[pt]; ph[u] = phi[pt];
+		st[u] = sqrt((1.0 - x[u]) * (1.0 + x[u]));
+		pow_ext(st[u], dA * p.mres, stA[u], eA[u]);
+		pow_ext(st[u], dB * p.mres, stB[u], eB[u]);
+		sincos_mul((double)(dA * p.mres), ph[u], rsA[u], rcA[u]);
+		sincos_mul((double)(dB * p.mres), ph[u], rsB[u], rcB[u]);
+		sp[u] = 0.0; spE[u] = 0; cs[u] = 1.0; sn[u] = 0.0;
+		#pragma unroll
+		for (int c = 0; c < NC; c++) v[u][c] = 0.0;
+	}
+	bool have = false;                        // sp holds sin^(m-1) of this warp's last order
+	for (int i = 0; i * W <= p.mtr; i++) {
+		const int im = i * W + ((i & 1) ? W - 1 - w : w);
+		const bool use = im <= p.mtr;
+		const int m = im * p.mres;
+		if (!use || m > p.ltr) break;         // later rounds only hold higher orders
+		const double2* al = reinterpret_cast<const double2*>(p.alm + p.almoff[im]);   // (c_m, a_{m+1}), (b_l, a_l) ...
+		const long j0 = lm_index(p, im, m);
+		const double2 *Q = p.Q ? p.Q + j0 : nullptr, *S = (NC == 3 && p.S) ? p.S + j0 : nullptr,
+		              *T = (NC == 3 && p.T) ? p.T + j0 : nullptr;
+		const double2 zero = make_double2(0.0, 0.0);
+		const double cm = al[0].x;
+		PtsState<NC> z[P];
+		double s2[P];
+		const int n = p.ltr - m;              // degrees beyond m
+		// bits by which the values can grow over the n steps: while they grow,
+		// P_l <= a_l P_{l-1} (b_l < 0 only takes away), a_l <= 2 sqrt(ltr / (l - m)),
+		// so by at most sqrt((4 ltr)^n / n!), and n! >= (n / e)^n
+		const float grow = n > 0 ? 0.5f * n * log2f(10.8732f * p.ltr / n) + 8.0f : 8.0f;
+		#pragma unroll
+		for (int u = 0; u < P; u++) {
+			int E = 0;
+			double y = 1.0;
+			if (m > 0) {
+				if (!have) pow_ext(st[u], m - 1, sp[u], spE[u]);
+				else {
+					sp[u] *= (i & 1) ? stA[u] : stB[u];
+					spE[u] += (i & 1) ? eA[u] : eB[u];
+					if (sp[u] < 0x1p-300 && sp[u] > 0.0) { sp[u] *= 0x1p300; spE[u] -= 300; }
+				}
+				y = sp[u]; E = spE[u];
+			}
+			y *= cm;
+			if (E >= -LOC_FOLD) { y = ldexp(y, E); E = 0; }
+			else if ((float) E + grow < -200.0f) { y = 0.0; E = 0; }      // no degree kept of this order can matter here
+			z[u].E = E;
+			z[u].y0 = 0.0; z[u].y1 = y;
+			z[u].d0 = 0.0; z[u].d1 = (m > 0) ? x[u] * m * y : 0.0;
+			z[u].q = z[u].sdt = z[u].tdt = z[u].sy = z[u].ty = zero;
+			s2[u] = (m > 0) ? st[u] * st[u] : st[u];
+			// e^(i m phi)
+			if (i % PTS_ROT == 0) sincos_mul((double) m, ph[u], sn[u], cs[u]);
+			else {
+				const double rc = (i & 1) ? rcA[u] : rcB[u], rs = (i & 1) ? rsA[u] : rsB[u];
+				const double c0 = cs[u];
+				cs[u] = fma(c0, rc, -sn[u] * rs);
+				sn[u] = fma(c0, rs, sn[u] * rc);
+			}
+		}
+		have = m > 0;
+		auto add = [&](auto G, double2 q, double2 s, double2 t) {
+			#pragma unroll
+			for (int u = 0; u < P; u++) pts_add<NC, decltype(G)::value>(z[u], q, s, t);
+		};
+		auto step = [&](double2 ba) {            // to the next degree
+			#pragma unroll
+			for (int u = 0; u < P; u++) {
+				const double y2 = ba.y * (x[u] * z[u].y1) + ba.x * z[u].y0;      // pair 0: z.y0 = 0
+				if constexpr (NC == 3) {
+					const double d2 = ba.y * (x[u] * z[u].d1 - s2[u] * z[u].y1) + ba.x * z[u].d0;
+					z[u].d0 = z[u].d1; z[u].d1 = d2;
+				}
+				z[u].y0 = z[u].y1; z[u].y1 = y2;
+			}
+		};
+		// chunks of 32 degrees: lane i brings what degree m + j0 + i needs, one
+		// chunk ahead, and the warp reads it back from its own shared buffers.
+		// Degrees beyond n are zeros, which leave the sums as they are.
+		double2 nx[NV];
+		auto fetch = [&](int j0) {
+			const int j = j0 + lane;
+			const bool in = j <= n;
+			nx[0] = in ? __ldg(al + j - 1) : zero;
+			nx[1] = (in && Q) ? __ldg(Q + j) : zero;
+			if constexpr (NC == 3) {
+				nx[2] = (in && S) ? __ldg(S + j) : zero;
+				nx[3] = (in && T) ? __ldg(T + j) : zero;
+			}
+		};
+		add(std::true_type{}, Q ? __ldg(Q) : zero, S ? __ldg(S) : zero, T ? __ldg(T) : zero);
+		if (n > 0) fetch(1);
+		for (int j0 = 1, c = 0; j0 <= n; j0 += 32, c ^= 1) {
+			double2 (*buf)[NV] = stage + 32 * c;
+			#pragma unroll
+			for (int v2 = 0; v2 < NV; v2++) buf[lane][v2] = nx[v2];
+			__syncwarp();
+			if (j0 + 32 <= n) fetch(j0 + 32);
+			const int nb = (min(32, n + 1 - j0) + 7) / 8;
+			for (int b = 0; b < nb; b++) {
+				const double2 (*r)[NV] = buf + 8 * b;
+				bool any = false;
+				#pragma unroll
+				for (int u = 0; u < P; u++) any = any || z[u].E != 0;
+				if (__any_sync(0xffffffffu, any)) {
+					#pragma unroll 1
+					for (int k = 0; k < 8; k++) { step(r[k][0]); add(std::true_type{}, r[k][1], r[k][NV > 2 ? 2 : 0], r[k][NV > 2 ? 3 : 0]); }
+					#pragma unroll
+					for (int u = 0; u < P; u++)
+						if (z[u].E && fabs(z[u].y1) > PTS_BIG) {
+							const int e = (z[u].E >= -LOC_FOLD - 400) ? z[u].E : -400;
+							z[u].y0 = ldexp(z[u].y0, e); z[u].y1 = ldexp(z[u].y1, e);
+							z[u].d0 = ldexp(z[u].d0, e); z[u].d1 = ldexp(z[u].d1, e);
+							z[u].E -= e;
+						}
+				} else {
+					#pragma unroll
+					for (int k = 0; k < 8; k++) { step(r[k][0]); add(std::false_type{}, r[k][1], r[k][NV > 2 ? 2 : 0], r[k][NV > 2 ? 3 : 0]); }
+				}
+			}
+			__syncwarp();
+		}
+		#pragma unroll
+		for (int u = 0; u < P; u++) {
+			const double c2 = im ? 2.0 : 1.0, sr = (m > 0) ? st[u] : 1.0;
+			const double C = c2 * cs[u], D = c2 * sn[u];
+			v[u][0] += (z[u].q.x * sr) * C - (m > 0 ? (z[u].q.y * sr) * D : 0.0);
+			if constexpr (NC == 3) {
+				// F_t = i m sum y T + sum dy S, F_p = i m sum y S - sum dy T (m = 0: real parts)
+				const double tr = z[u].sdt.x - m * z[u].ty.y, ti = z[u].sdt.y + m * z[u].ty.x;
+				const double pr = -z[u].tdt.x - m * z[u].sy.y, pi = -z[u].tdt.y + m * z[u].sy.x;
+				v[u][1] += tr * C - (m > 0 ? ti * D : 0.0);
+				v[u][2] += pr * C - (m > 0 ? pi * D : 0.0);
+			}
+		}
+	}
+	constexpr int PC = 32 * P;
+	double* red = reinterpret_cast<double*>(pts_smem);      // [warp][component][point of the CTA]
+	__syncthreads();
+	#pragma unroll
+	for (int u = 0; u < P; u++)
+		#pragma unroll
+		for (int c = 0; c < NC; c++) red[(w * NC + c) * PC + u * 32 + lane] = v[u][c];
+	__syncthreads();
+	for (int e = threadIdx.x; e < NC * PC; e += blockDim.x) {
+		const int c = e / PC, i = e - c * PC, pt = blockIdx.x * PC + i;
+		if (pt >= npts) continue;
+		double sum = 0.0;
+		for (int k = 0; k < W; k++) sum += red[(k * NC + c) * PC + i];
+		(c == 0 ? o0 : c == 1 ? o1 : o2)[pt] = sum;
 	}
 }
 
@@ -533,14 +769,40 @@ extern "C" void SH_mul_mx(shtns_cfg s, double* mx, cplx* Qlm, cplx* Rlm)
 }
 
 // ---- batched device forms (no counterpart in the reference) ----
+namespace {
+
+// Points per lane and warps per CTA.  Two points per lane (independent
+// chains) once that leaves every SM work; enough warps per CTA for about 24 per SM.
+// Fewer than 256 points fill less than eight warps: those keep a CTA each (a
+// lane per order).  255 and 256 points: lmax 127 73 and 45 us, 255 159 and 142,
+// 1023 2266 and 2296.
+template <int NC>
+void launch_points(shtns_cfg s, const LocalParams& p, const double* cost, const double* phi, int npts,
+                   double* o0, double* o1, double* o2)
+{
+	if (npts < 256) {
+		point_kernel<<<npts, PT_THREADS, 0, s->comp_stream>>>(p, cost, phi, NC, 0, o0, o1, o2);
+	} else {
+		const bool two = NC == 1 && npts >= 64 * 148;
+		const int tiles = two ? (npts + 63) / 64 : (npts + 31) / 32;
+		int W = 4;
+		while (W < (NC == 3 ? 8 : 16) && (long) tiles * W < 24 * 148 && 2 * W <= p.mtr + 1) W *= 2;
+		const size_t smem = sizeof(double2) * 64 * W * (NC == 3 ? 4 : 2);    // the sums take less
+		if (two) points_kernel<NC, NC == 1 ? 2 : 1><<<tiles, 32 * W, smem, s->comp_stream>>>(p, cost, phi, npts, o0, o1, o2);
+		else points_kernel<NC, 1><<<tiles, 32 * W, smem, s->comp_stream>>>(p, cost, phi, npts, o0, o1, o2);
+	}
+	shtb_count_launch();
+	shtb_cuda_ok(cudaGetLastError(), "point evaluation launch");
+}
+
+} // namespace
+
 extern "C" void shtns_b200_SH_to_points(shtns_cfg s, cplx* Qlm, const double* cost, const double* phi, double* v, int npts)
 {
 	if (!loc_check(s) || npts <= 0) return;
 	LocalParams p = loc_params(s);
 	p.Q = reinterpret_cast<const double2*>(Qlm);
-	point_kernel<<<npts, PT_THREADS, 0, s->comp_stream>>>(p, cost, phi, 1, 0, v, nullptr, nullptr);
-	shtb_count_launch();
-	shtb_cuda_ok(cudaGetLastError(), "point evaluation launch");
+	launch_points<1>(s, p, cost, phi, npts, v, nullptr, nullptr);
 }
 
 extern "C" void shtns_b200_SHqst_to_points(shtns_cfg s, cplx* Qlm, cplx* Slm, cplx* Tlm, const double* cost,
@@ -551,7 +813,5 @@ extern "C" void shtns_b200_SHqst_to_points(shtns_cfg s, cplx* Qlm, cplx* Slm, cp
 	p.Q = reinterpret_cast<const double2*>(Qlm);
 	p.S = reinterpret_cast<const double2*>(Slm);
 	p.T = reinterpret_cast<const double2*>(Tlm);
-	point_kernel<<<npts, PT_THREADS, 0, s->comp_stream>>>(p, cost, phi, 3, 0, vr, vt, vp);
-	shtb_count_launch();
-	shtb_cuda_ok(cudaGetLastError(), "point evaluation launch");
+	launch_points<3>(s, p, cost, phi, npts, vr, vt, vp);
 }

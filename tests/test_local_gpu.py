@@ -206,3 +206,41 @@ def test_batched_points_equal_single_points():
     pp = torch.from_numpy((2 * np.pi * j / 432).ravel()).to(dev)
     v = sh.points(torch.from_numpy(q).to(dev), pc, pp).cpu().numpy()
     assert relerr(grid[i, j].ravel(), v) < TOL
+
+
+@pytest.mark.parametrize("lmax,mmax,mres", [(2, 2, 1), (31, 10, 3), (200, 200, 1), (700, 700, 1)])
+@pytest.mark.parametrize("npts", [1, 255, 256, 257, 1000, 64 * 148 - 1, 64 * 148 + 1])
+def test_many_points_equal_the_kernel_per_point(lmax, mmax, mres, npts):
+    """Calls of many points (a lane per point) against calls of few (a CTA per
+    point): scalar and vector values, with points at and near the poles, where
+    the high orders' seeds leave the double range.  The recurrence is the same;
+    the sums over orders and the phases e^(i m phi) are formed in another
+    order: lmax 2^-53 phi_max of the largest value, with a factor 4."""
+    import torch
+    import shtns_b200
+    dev = torch.device("cuda:0")
+    sh = shtns_b200.sht(lmax, mmax, mres)
+    rng = np.random.default_rng(npts + lmax)
+    ct = rng.uniform(-1, 1, npts)
+    edge = [1.0, -1.0, 0.0, 1 - 1e-16, 0.9999999, -0.999999, 0.999, -0.99]
+    ct[: len(edge)] = edge[:npts]
+    ph = rng.uniform(-np.pi, 2 * np.pi, npts)
+    c, p = torch.from_numpy(ct).to(dev), torch.from_numpy(ph).to(dev)
+    q, s, t = (torch.from_numpy(rand_spec(lmax, mmax, mres, 31 + i, power=1.0 + 0.5 * (i > 0), zero_l0=i > 0)).to(dev) for i in range(3))
+    pick = np.unique(np.concatenate([np.arange(min(npts, 40)), rng.integers(0, npts, 60)]))[:100]
+    tol = 4 * lmax * 2.0 ** -53 * 2 * np.pi
+    v = sh.points(q, c, p).cpu().numpy()
+    few = sh.points(q, c[pick], p[pick]).cpu().numpy()
+    assert np.abs(v[pick] - few).max() <= tol * np.abs(v).max()
+    sh._stream()
+
+    def vec(c, p, S):
+        out = [torch.full_like(c, float("nan")) for _ in range(3)]
+        sh._lib.shtns_b200_SHqst_to_points(sh._cfg, C.c_void_p(q.data_ptr()), C.c_void_p(S.data_ptr()) if S is not None else None,
+                                           C.c_void_p(t.data_ptr()), C.c_void_p(c.data_ptr()), C.c_void_p(p.data_ptr()),
+                                           *[C.c_void_p(o.data_ptr()) for o in out], int(c.numel()))
+        return [o.cpu().numpy() for o in out]
+    for S in (s, None):
+        a, b = vec(c, p, S), vec(c[pick].contiguous(), p[pick].contiguous(), S)
+        for x, y in zip(a, b):
+            assert np.abs(x[pick] - y).max() <= tol * max(np.abs(x).max(), 1e-300)
