@@ -91,58 +91,60 @@ __global__ void ck_kernel(int nlat_2, int mres, int seg, const double* __restric
 // Column layout: field-component fc owns columns 16*(fc/4) + 2*(fc%4) + {0,1}
 // (even re, im) and the same +8 (odd re, im).
 //
-// CTA = (order im, PT_K = pt_items / PF Ishioka rows k, PF field-components): the degree
-// window [2 k0 - 1, 2 k0 + 2 PT_K + 2] of each input array is staged in shared
-// memory with coalesced loads, then every qq row segment is written
-// contiguously.  PF is the power of two up to 16 that the call's
-// field-components fill best (launch_prep_synth): with 16 for every call, one
-// qst field at lmax 1023 kept 3 of 16 lanes and took 68 us instead of 35 (8
-// scalar fields at lmax 4095: 684 instead of 452).
-__host__ __device__ constexpr int pt_items(int PF) { return PF <= 2 ? 256 : 512; }     // (row, field-component) items of a CTA
+// CTA = (order im, PT_K = pt_items / PF Ishioka rows k, PF fields, group): the
+// first group is the scalar component, the other one the vector pair.  The
+// degree window [2 k0 - 1, 2 k0 + 2 PT_K + 2] of Q, or of S and T, is staged in
+// shared memory with coalesced loads; then each thread forms the rows of one
+// (k, field), for the vector pair V and W together from the same five degrees
+// of S and T.  PF is the power of two up to 16 that the call's fields fill best
+// (launch_prep_synth): with 16 for every call, one qst field at lmax 1023 kept 3
+// of 16 lanes and took 68 us instead of 35 (8 scalar fields at lmax 4095: 684
+// instead of 452).  Bound: instruction issue and the shared-memory path.  With V
+// and W as field-components of their own, S and T were staged twice and read
+// 18 instead of 10 times per pair (64 qst fields
+// at lmax 511: 241 us, here 195; 32 vector fields at lmax 255: 33, here 28).
+__host__ __device__ constexpr int pt_items(int PF) { return PF <= 2 ? 256 : 512; }     // (row, field) items of a CTA
 
 // C: coefficient type, double2, or float2 for the single-precision transforms.
-template <int PF, class C>
-__global__ void __launch_bounds__(256, 6) prep_synth_kernel(PrepParams p)
+// VECTOR: the call has a vector pair (and perhaps a scalar component).
+template <int PF, class C, bool VECTOR>
+__global__ void __launch_bounds__(256, VECTOR ? 4 : 6) prep_synth_kernel(PrepParams p)
 {
 	constexpr int PT_F = PF, PT_K = pt_items(PF) / PF;
 	constexpr int PT_W = 2 * PT_K + 5;       // window length, odd stride in 16-byte units
-	__shared__ double2 win[2][PT_F][PT_W];
-	__shared__ double cfs[2][PT_W];          // sin d/dtheta coupling (lo, hi) of the window's degrees
+	constexpr int NA = VECTOR ? 2 : 1;       // arrays staged
+	__shared__ double2 win[NA][PT_F][PT_W];
+	__shared__ double cfs[NA][PT_W];         // sin d/dtheta coupling (lo, hi) of the window's degrees
 	__shared__ double xk[3 * PT_K];          // basis change X of the CTA's k rows
-	__shared__ int s_comp[PT_F], s_f[PT_F];
 	const int im = p.im0 + blockIdx.z;
 	if (im > p.mlim) return;
 	const int m = im * p.mres;
 	const int kmax = (p.llim + 1 - m) / 2 + 1;
 	const int k0 = blockIdx.x * PT_K;
 	if (k0 >= kmax) return;
-	const int nfc = p.nf * p.ncomp;
-	const int fc0 = blockIdx.y * PT_F;
+	const bool has_q = p.comp_type[0] == 0;
+	const int nft = (p.nf + PT_F - 1) / PT_F;
+	const int grp = blockIdx.y / nft;
+	const int f0 = (blockIdx.y - grp * nft) * PT_F;
+	const bool vec = VECTOR && !(has_q && grp == 0);
 	const bool m0 = (m == 0);
 	const int lrel_max = p.llim - m;
 	const long off = (long)im * (2 * p.lmax + 2 - (im + 1) * p.mres) / 2 + m;   // LM(m, m)
 	const int d0 = 2 * k0 - 1;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int voff = p.mt.voff[im];
-	const bool vec = p.comp_type[0] != 0 || p.ncomp > 1;
-	if (tid < PT_F) {
-		const int fc = fc0 + tid;
-		const int comp = fc / p.nf;
-		s_comp[tid] = (fc < nfc) ? comp : -1;
-		s_f[tid] = fc - comp * p.nf;
-	}
 	if (vec)
 		for (int i = tid; i < PT_W; i += 256) {
 			const int d = d0 + i;
 			cfs[0][i] = (d > 0 && d <= lrel_max + 1) ? p.stdt_lo[voff + d] : 0.0;
-			cfs[1][i] = (d >= 0 && d <= lrel_max + 1) ? p.stdt_hi[voff + d] : 0.0;
+			cfs[NA - 1][i] = (d >= 0 && d <= lrel_max + 1) ? p.stdt_hi[voff + d] : 0.0;
 		}
 	for (int e = tid; e < 3 * PT_K; e += 256) xk[e] = (k0 + e / 3 <= kmax) ? p.xs[p.mt.xoff[im] + 3 * k0 + e] : 0.0;
-	// window of the degrees of each (array, field-component) pair (array =
-	// pair / PF, the second one for vectors only), lanes along the degrees: WP
-	// warps share a pair or a warp takes PW of them, QB pairs and up to UB loads
-	// of each before the first store
-	constexpr int WP = (2 * PF >= 8) ? 1 : 8 / (2 * PF), PW = (2 * PF >= 8) ? 2 * PF / 8 : 1;
+	// window of the degrees of each (array, field) pair (array = pair / PF, the
+	// second one for vectors only), lanes along the degrees: WP warps share a
+	// pair or a warp takes PW of them, QB pairs and up to UB loads of each before
+	// the first store
+	constexpr int NP = NA * PF, WP = (NP >= 8) ? 1 : 8 / NP, PW = (NP >= 8) ? NP / 8 : 1;
 	constexpr int NI = (PT_W + 32 * WP - 1) / (32 * WP);
 	constexpr int QB = (PW >= 2 && NI <= 3) ? 2 : 1, UB = (NI <= 5) ? NI : (NI + 1) / 2;
 	const int q0 = (WP == 1) ? warp : warp / WP, i0 = lane + 32 * (warp % WP);
@@ -151,13 +153,9 @@ __global__ void __launch_bounds__(256, 6) prep_synth_kernel(PrepParams p)
 		const C* base[QB];
 		#pragma unroll
 		for (int qi = 0; qi < QB; qi++) {
-			const int q = q0 + 8 * (h + qi), a = q / PT_F, fc = fc0 + q % PT_F;
-			base[qi] = nullptr;
-			if (fc < nfc && (a == 0 || vec)) {
-				const int comp = fc / p.nf, f = fc - comp * p.nf;
-				const double2* x = (p.comp_type[comp] == 0) ? (a == 0 ? p.Q : nullptr) : (a == 0 ? p.S : p.T);
-				if (x) base[qi] = reinterpret_cast<const C*>(x) + off + (long)f * p.spec_dist + d0;
-			}
+			const int q = q0 + 8 * (h + qi), a = q / PT_F, f = f0 + q % PT_F;
+			const double2* x = vec ? (a == 0 ? p.S : p.T) : (a == 0 ? p.Q : nullptr);
+			base[qi] = (x && f < p.nf) ? reinterpret_cast<const C*>(x) + off + (long)f * p.spec_dist + d0 : nullptr;
 		}
 		#pragma unroll
 		for (int u0 = 0; u0 < NI; u0 += UB) {
@@ -176,7 +174,7 @@ __global__ void __launch_bounds__(256, 6) prep_synth_kernel(PrepParams p)
 			#pragma unroll
 			for (int qi = 0; qi < QB; qi++) {
 				const int q = q0 + 8 * (h + qi), a = q / PT_F, fl = q % PT_F;
-				if (a != 0 && !vec) continue;
+				if (VECTOR && a != 0 && !vec) continue;
 				#pragma unroll
 				for (int u = 0; u < UB; u++) {
 					const int i = i0 + 32 * WP * (u0 + u);
@@ -187,40 +185,41 @@ __global__ void __launch_bounds__(256, 6) prep_synth_kernel(PrepParams p)
 	}
 	__syncthreads();
 	const double em = (p.msign < 0) ? -(double) m : (double) m;   // signed m (negative orders of the _ml transforms)
+	const long row0 = p.mt.koff[im];
+	// even and odd parts of field-component fc at row k from its degrees 2k .. 2k + 2
+	auto put = [&](int k, int fc, const double* x, double2 a, double2 b, double2 c) {
+		double* row = p.qq + (row0 + k) * p.ncol + 16 * (fc >> 2) + 2 * (fc & 3);
+		*reinterpret_cast<double2*>(row) = make_double2(fma(x[0], a.x, x[1] * c.x), fma(x[0], a.y, x[1] * c.y));
+		*reinterpret_cast<double2*>(row + 8) = make_double2(x[2] * b.x, x[2] * b.y);
+	};
 	for (int e = tid; e < PT_K * PT_F; e += 256) {
 		const int kl = e / PT_F, fl = e - kl * PT_F;
-		const int k = k0 + kl, fc = fc0 + fl;
-		if (k >= kmax || fc >= nfc) continue;
-		const int type = p.comp_type[s_comp[fl]];
-		// fields from neg_from on carry the order -m (complex-field transforms)
-		const int fld = s_f[fl];
-		const double emf = (p.neg_from > 0 && fld >= p.neg_from) ? -em : em;
-		const int i0 = 2 * kl + 1;                 // window index of degree 2k
-		double2 q3[3];
-		if (type == 0) {
-			#pragma unroll
-			for (int r = 0; r < 3; r++) q3[r] = win[0][fl][i0 + r];
-		} else {
-			// V = stdt S + i m T (type 1), W = -stdt T + i m S (type 2): the
-			// coupled array at degrees d -/+ 1, the other one at d
-			const int ac = (type == 1) ? 0 : 1;
-			#pragma unroll
-			for (int r = 0; r < 3; r++) {
-				const int d = 2 * k + r;               // relative degree
-				if (d > lrel_max + 1) { q3[r] = make_double2(0.0, 0.0); continue; }
-				const double lo = cfs[0][i0 + r], hi = cfs[1][i0 + r];
-				const double2 cm = win[ac][fl][i0 - 1 + r], cp = win[ac][fl][i0 + 1 + r], o0 = win[1 - ac][fl][i0 + r];
-				if (type == 1)
-					q3[r] = make_double2(lo * cm.x + hi * cp.x - emf * o0.y, lo * cm.y + hi * cp.y + emf * o0.x);
-				else
-					q3[r] = make_double2(-(lo * cm.x + hi * cp.x) - emf * o0.y, -(lo * cm.y + hi * cp.y) + emf * o0.x);
-			}
+		const int k = k0 + kl, f = f0 + fl;
+		if (k >= kmax || f >= p.nf) continue;
+		const int w0 = 2 * kl;                     // window index of degree 2k - 1
+		const double* x = xk + 3 * kl;
+		if (!vec) {
+			put(k, f, x, win[0][fl][w0 + 1], win[0][fl][w0 + 2], win[0][fl][w0 + 3]);
+			continue;
 		}
-		const double x0 = xk[3 * kl], x1 = xk[3 * kl + 1], x2 = xk[3 * kl + 2];
-		double* row = p.qq + (long)(p.mt.koff[im] + k) * p.ncol;
-		const int ce = 16 * (fc >> 2) + 2 * (fc & 3);
-		*reinterpret_cast<double2*>(row + ce) = make_double2(fma(x0, q3[0].x, x1 * q3[2].x), fma(x0, q3[0].y, x1 * q3[2].y));
-		*reinterpret_cast<double2*>(row + ce + 8) = make_double2(x2 * q3[1].x, x2 * q3[1].y);
+		// V = stdt S + i m T, W = -stdt T + i m S: the coupled array at degrees
+		// d -/+ 1, the other one at d (zero beyond lrel_max + 1, where the
+		// coupling is zero and so are S and T).  Fields from neg_from on carry the
+		// order -m (complex-field transforms)
+		const double emf = (p.neg_from > 0 && f >= p.neg_from) ? -em : em;
+		double2 s[5], t[5];
+		#pragma unroll
+		for (int r = 0; r < 5; r++) { s[r] = win[0][fl][w0 + r]; t[r] = win[NA - 1][fl][w0 + r]; }
+		double2 v[3], w[3];
+		#pragma unroll
+		for (int r = 0; r < 3; r++) {
+			const double lo = cfs[0][w0 + 1 + r], hi = cfs[NA - 1][w0 + 1 + r];
+			v[r] = make_double2(lo * s[r].x + hi * s[r + 2].x - emf * t[r + 1].y, lo * s[r].y + hi * s[r + 2].y + emf * t[r + 1].x);
+			w[r] = make_double2(-(lo * t[r].x + hi * t[r + 2].x) - emf * s[r + 1].y, -(lo * t[r].y + hi * t[r + 2].y) + emf * s[r + 1].x);
+		}
+		const int fv = (has_q ? p.nf : 0) + f;
+		put(k, fv, x, v[0], v[1], v[2]);
+		put(k, fv + p.nf, x, w[0], w[1], w[2]);
 	}
 }
 
@@ -451,7 +450,7 @@ void launch_checkpoints(shtns_cfg s, cudaStream_t st)
 	cudaFree(d_nseg);
 }
 
-// Fields (or field-components) per CTA of the prologue and epilogue kernels: 1
+// Fields per CTA of the prologue and epilogue kernels: 1
 // or 2 for so many, else the largest of 16, 8 and 4 that leaves the fewest
 // idle (fewer than 4 split the 64-byte groups of four field-components)
 static int tile_fields(int n)
@@ -465,25 +464,28 @@ static int tile_fields(int n)
 
 void launch_prep_synth(const PrepParams& p, cudaStream_t st)
 {
-	const int nfc = p.nf * p.ncomp;
+	const int ngroups = (p.comp_type[0] == 0) ? 1 + (p.ncomp > 1 ? 1 : 0) : 1;
 	const int kmax0 = (p.llim + 1) / 2 + 1;
 	auto go = [&](auto kern, int PF) {
 		const int K = pt_items(PF) / PF;
-		dim3 grid((kmax0 + K - 1) / K, (nfc + PF - 1) / PF, p.mlim + 1 - p.im0);
+		dim3 grid((kmax0 + K - 1) / K, (p.nf + PF - 1) / PF * ngroups, p.mlim + 1 - p.im0);
 		kern<<<grid, 256, 0, st>>>(p);
 	};
-	auto pick = [&](auto c) {
+	auto pick = [&](auto c, auto VC) {
 		using C = decltype(c);
-		switch (tile_fields(nfc)) {
-			case 1: go(prep_synth_kernel<1, C>, 1); break;
-			case 2: go(prep_synth_kernel<2, C>, 2); break;
-			case 4: go(prep_synth_kernel<4, C>, 4); break;
-			case 8: go(prep_synth_kernel<8, C>, 8); break;
-			default: go(prep_synth_kernel<16, C>, 16); break;
+		constexpr bool V = decltype(VC)::value;
+		switch (tile_fields(p.nf)) {
+			case 1: go(prep_synth_kernel<1, C, V>, 1); break;
+			case 2: go(prep_synth_kernel<2, C, V>, 2); break;
+			case 4: go(prep_synth_kernel<4, C, V>, 4); break;
+			case 8: go(prep_synth_kernel<8, C, V>, 8); break;
+			default: go(prep_synth_kernel<16, C, V>, 16); break;
 		}
 	};
-	if (p.f32) pick(float2{});
-	else pick(double2{});
+	const bool vector = ngroups > 1 || p.comp_type[0] != 0;
+	if (p.f32) pick(float2{}, std::false_type{});      // single-precision transforms are scalar
+	else if (vector) pick(double2{}, std::true_type{});
+	else pick(double2{}, std::false_type{});
 	shtb_count_launch();
 }
 
