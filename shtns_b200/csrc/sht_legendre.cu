@@ -241,35 +241,29 @@ template <int PF>
 struct PostTile {
 	static constexpr int J = (PF == 1) ? 512 : (PF == 4) ? 128 : 1024 / PF;   // degrees
 	static constexpr int R = J / 2 + 4;                     // staged k rows: j0/2-2 .. j0/2+J/2+1
-	static constexpr int S = (PF == 1) ? 2 : 2 * PF + 2;    // row stride in double2: 32 mod 128 bytes, so the 4 rows read by 8 lanes use distinct banks
+	static constexpr int S = 2 * PF + 1;                    // row stride in double2: odd, so the 8 rows read by 8 lanes use distinct banks
 };
 
-// E[row][2 fl + 0] = even pair (re, im), [2 fl + 1] = odd pair, row = k - kb;
-// Xs[3 row + c] = basis-change coefficients of k
+// Staged rows: [row][2 fl] = even pair (re, im) of field fl, [2 fl + 1] = odd
+// pair, row = k - kb; Xs[3 row + c] = basis-change coefficients of k (both zero
+// outside the order).  Degree 2k, and degree 2k + 1:
 template <int PE_S>
-__device__ __forceinline__ double2 ish_inv_s(const double2 (*E)[PE_S], const double* Xs, int kb, int fl, int j)
+__device__ __forceinline__ double2 ish_even(const double2 (*E)[PE_S], const double* Xs, int r, int fl)
 {
-	if (j < 0) return make_double2(0.0, 0.0);
-	const int r = (j >> 1) - kb;
-	if ((j & 1) == 0) {
-		const double2 e = E[r][2 * fl];
-		const double x = Xs[3 * r];
-		double2 q = make_double2(x * e.x, x * e.y);
-		if (j > 1) {
-			const double2 e1 = E[r - 1][2 * fl];
-			const double x1 = Xs[3 * (r - 1) + 1];
-			q.x = fma(x1, e1.x, q.x);
-			q.y = fma(x1, e1.y, q.y);
-		}
-		return q;
-	}
+	const double2 e = E[r][2 * fl], e1 = E[r - 1][2 * fl];
+	const double x = Xs[3 * r], x1 = Xs[3 * (r - 1) + 1];
+	return make_double2(fma(x1, e1.x, x * e.x), fma(x1, e1.y, x * e.y));
+}
+template <int PE_S>
+__device__ __forceinline__ double2 ish_odd(const double2 (*E)[PE_S], const double* Xs, int r, int fl)
+{
 	const double2 o = E[r][2 * fl + 1];
-	const double x2 = Xs[3 * r + 2];
-	return make_double2(x2 * o.x, x2 * o.y);
+	const double x = Xs[3 * r + 2];
+	return make_double2(x * o.x, x * o.y);
 }
 
 template <int PF, class C>
-__global__ void __launch_bounds__(256) post_analys_kernel(PrepParams p)
+__global__ void __launch_bounds__(256, 4) post_analys_kernel(PrepParams p)
 {
 	constexpr int PE_F = PF, PE_J = PostTile<PF>::J, PE_R = PostTile<PF>::R, PE_S = PostTile<PF>::S;
 	constexpr int NE = PE_R * PE_F * 2, NU = (NE + 255) / 256;
@@ -344,57 +338,57 @@ __global__ void __launch_bounds__(256) post_analys_kernel(PrepParams p)
 	}
 	__syncthreads();
 	const double em = (p.msign < 0) ? -(double) m : (double) m;   // signed m (negative orders of the _ml transforms)
-	const int lane = threadIdx.x & 31;
 	auto store = [&](double2* to, long at, double2 v) {
 		C x;
 		x.x = v.x; x.y = v.y;
 		reinterpret_cast<C*>(to)[at] = x;
 	};
-	// a warp covers 32 consecutive degrees of one field: each lane forms its
-	// own degree in the spectral basis and takes the neighbours (j -/+ 1) of
-	// the vector formulas from the adjacent lanes
-	for (int e = threadIdx.x; e < PE_J * PE_F; e += blockDim.x) {
-		const int fl = e / PE_J, jl = e - fl * PE_J;
-		const int j = j0 + jl, f = f0 + fl;
-		const int l = m + j;
-		const bool live = j < nl && f < p.nf;
+	// an item is a pair of degrees (2k, 2k + 1) of one field, 32 consecutive k to
+	// a warp: the four degrees 2k - 1 .. 2k + 2 that its vector formulas need come
+	// from five staged values per array (one degree per item read twice as much of
+	// the shared-memory path: 64 qst fields at lmax 511 206 us, here 183; 32 scalar
+	// fields at lmax 1023 140, here 132; 32 vector fields at lmax 255 27, here 23)
+	for (int e = threadIdx.x; e < PE_J / 2 * PE_F; e += blockDim.x) {
+		const int fl = e / (PE_J / 2), i = e - fl * (PE_J / 2), r = i + 2;
+		const int j = j0 + 2 * i, f = f0 + fl;
+		if (j >= nl || f >= p.nf) continue;
+		const bool two = j + 1 < nl;
+		const bool z0 = zero_m || m + j > p.llim, z1 = zero_m || m + j + 1 > p.llim;
 		const long o = off + (long)f * p.spec_dist + j;
-		const bool zero = zero_m || (l > p.llim);
+		double2 s0 = make_double2(0.0, 0.0), s1 = s0, t0 = s0, t1 = s0;
 		if (scalar_group) {
-			if (!live) continue;
-			double2 q = make_double2(0.0, 0.0);
-			if (!zero) {
-				q = ish_inv_s(sv, xs, kb, fl, j);
-				if (m == 0) q.y = 0.0;
+			if (!z0) {
+				s0 = ish_even(sv, xs, r, fl);
+				if (m == 0) s0.y = 0.0;
 			}
-			store(p.Qo, o, q);
+			if (!z1) {
+				s1 = ish_odd(sv, xs, r, fl);
+				if (m == 0) s1.y = 0.0;
+			}
+			store(p.Qo, o, s0);
+			if (two) store(p.Qo, o + 1, s1);
 			continue;
 		}
-		const bool fv = !zero_m && f < p.nf && j < nl + 1;   // rows staged: degrees up to nl
-		const double2 v0 = fv ? ish_inv_s(sv, xs, kb, fl, j) : make_double2(0.0, 0.0);
-		const double2 w0 = fv ? ish_inv_s(sw, xs, kb, fl, j) : make_double2(0.0, 0.0);
-		double2 vm, vp, wm, wp;
-		vm.x = __shfl_up_sync(0xffffffffu, v0.x, 1); vm.y = __shfl_up_sync(0xffffffffu, v0.y, 1);
-		wm.x = __shfl_up_sync(0xffffffffu, w0.x, 1); wm.y = __shfl_up_sync(0xffffffffu, w0.y, 1);
-		vp.x = __shfl_down_sync(0xffffffffu, v0.x, 1); vp.y = __shfl_down_sync(0xffffffffu, v0.y, 1);
-		wp.x = __shfl_down_sync(0xffffffffu, w0.x, 1); wp.y = __shfl_down_sync(0xffffffffu, w0.y, 1);
-		if (!live) continue;
-		double2 s = make_double2(0.0, 0.0), t = make_double2(0.0, 0.0);
-		if (!zero) {
-			if (lane == 0) { vm = ish_inv_s(sv, xs, kb, fl, j - 1); wm = ish_inv_s(sw, xs, kb, fl, j - 1); }
-			if (lane == 31) { vp = ish_inv_s(sv, xs, kb, fl, j + 1); wp = ish_inv_s(sw, xs, kb, fl, j + 1); }
-			const double lo = vlo[jl + 1];
-			const double hi = vhi[jl + 1];
-			const double l2 = vl2[jl];
-			const double mxv_r = lo * vm.x + hi * vp.x, mxv_i = lo * vm.y + hi * vp.y;
-			const double mxw_r = lo * wm.x + hi * wp.x, mxw_i = lo * wm.y + hi * wp.y;
+		if (!z0) {
 			const double emf = (p.neg_from > 0 && f >= p.neg_from) ? -em : em;   // order -m fields
-			s = make_double2(-(mxv_r - emf * w0.y) * l2, -(mxv_i + emf * w0.x) * l2);
-			t = make_double2(-(-emf * v0.y - mxw_r) * l2, -(emf * v0.x - mxw_i) * l2);
-			if (m == 0) { s.y = 0.0; t.y = 0.0; }
+			const double2 v[4] = {ish_odd(sv, xs, r - 1, fl), ish_even(sv, xs, r, fl), ish_odd(sv, xs, r, fl), ish_even(sv, xs, r + 1, fl)};
+			const double2 w[4] = {ish_odd(sw, xs, r - 1, fl), ish_even(sw, xs, r, fl), ish_odd(sw, xs, r, fl), ish_even(sw, xs, r + 1, fl)};
+			#pragma unroll
+			for (int h = 0; h < 2; h++) {
+				const double lo = vlo[2 * i + h + 1], hi = vhi[2 * i + h + 1], l2 = vl2[2 * i + h];
+				const double2 v0 = v[h + 1], w0 = w[h + 1];
+				const double mxv_r = lo * v[h].x + hi * v[h + 2].x, mxv_i = lo * v[h].y + hi * v[h + 2].y;
+				const double mxw_r = lo * w[h].x + hi * w[h + 2].x, mxw_i = lo * w[h].y + hi * w[h + 2].y;
+				double2 a = make_double2(-(mxv_r - emf * w0.y) * l2, -(mxv_i + emf * w0.x) * l2);
+				double2 b = make_double2(-(-emf * v0.y - mxw_r) * l2, -(emf * v0.x - mxw_i) * l2);
+				if (m == 0) { a.y = 0.0; b.y = 0.0; }
+				if (h == 0) { s0 = a; t0 = b; }
+				else if (!z1) { s1 = a; t1 = b; }
+			}
 		}
-		store(p.So, o, s);
-		store(p.To, o, t);
+		store(p.So, o, s0);
+		store(p.To, o, t0);
+		if (two) { store(p.So, o + 1, s1); store(p.To, o + 1, t1); }
 	}
 }
 
