@@ -85,8 +85,9 @@ int shtns_b200_transform(shtns_cfg, cudaStream_t stream, int howmany, int kind, 
                          void *e, void *f, int ltr);
 
 /* Tuning options of a plan.  option 1: latitude pairs per FFT CTA (1, 2, 4,
- * 8 where the fused chain's buffer fits; 0 = automatic); option 2: recurrence checkpoint spacing (8, 16, 32; rebuilds
- * the checkpoint table; not for clones or plans that have clones); option 3:
+ * 8 where the buffer fits; 0 = automatic); option 2: spacing of the recurrence
+ * checkpoint table (8, 16, 32; rebuilds the table, of which a kernel may use
+ * every second or fourth; not for clones or plans that have clones); option 3:
  * FFT kernels, 0 = automatic (for nphi = 3 * 2^k up to 3072: persistent CTAs
  * that prefetch their next latitude tile with tensor copies while the current
  * one is transformed, and on theta-contiguous grids write whole synthesis
@@ -102,7 +103,8 @@ int shtns_b200_transform(shtns_cfg, cudaStream_t stream, int howmany, int kind, 
  * (test hook, set only, any plan): fills the static scratch array of
  * cu_SH_to_spat_noalloc on the current device with the byte value 0..255
  * (0xFF: NaN doubles) and waits for it.  Option 10: FP64 Legendre values
- * of the 64 x 64 tile synthesis, 0 (default) from a table of Y_k(theta)
+ * of the 64 x 64 tile synthesis, 0 (default) for calls of more than 32
+ * field-components from a table of Y_k(theta)
  * built on the device on first use when it takes at most a quarter of the
  * free device memory and 8 GiB (about 0.2 GB at lmax 511 on 768 latitudes;
  * otherwise, and inside a stream capture before the table exists, on the
@@ -117,9 +119,11 @@ int shtns_b200_get_option(shtns_cfg, int option);
  * along the rows: 1 = 32 rows x 128 columns, 2 = 64 x 64, 4 = 128 x 32,
  * 8 = SIMT kernels (FP64 FMA, recurrence in registers; calls with 1 to 4
  * field-components, others fall back to the automatic choice); 0 (default)
- * picks the SIMT kernels for at most 4 field-components in the synthesis and
- * 3 in the analysis, 128 x 32 for calls with at most 32 GEMM columns (8
- * field-components) and 64 x 64 otherwise.  Plan groups always use 64 x 64.
+ * picks the SIMT kernels for the analysis of one field-component and the
+ * synthesis of one or two (three on grids of more than 1024 rows), 128 x 16
+ * tiles otherwise up to 4 (128 x 32 in the analysis up to 512 rows), 128 x 32
+ * up to 32 GEMM columns (8 field-components) and 64 x 64 beyond.  The
+ * persistent launch of plan groups always uses 64 x 64.
  * Option 4 of shtns_b200_set_option: split-precision Legendre stages with 3
  * to 7 balanced 8-bit digits per operand (products summed exactly; the
  * result carries about 8 x digits - 2 bits relative to the row and column
@@ -143,14 +147,14 @@ int shtns_b200_kernel_errors(shtns_cfg);
 size_t shtns_b200_split_table_bytes(shtns_cfg);
 
 /* Plan groups: transforms of fields of different lmax (scalar, and the vector
- * forms below), each on the grid
- * of its own plan, with the Legendre stage of all plans in one persistent
- * launch whose CTAs take work items (plan, order, tile) from a queue in
- * decreasing cost order.  Qlm[i] / Vr[i] hold nfields[i] contiguous fields of
+ * forms below), each on the grid of its own plan, every plan's kernels
+ * chained on a side stream of the group (or, option 5 = 0, with the Legendre
+ * stage of all plans in one persistent launch whose CTAs take work items (plan,
+ * order, tile) from a queue in decreasing cost order).  Qlm[i] / Vr[i] hold nfields[i] contiguous fields of
  * plan i (device pointers; spec_dist = nlm, spat_dist = nspat of that plan).
- * All launches go to the compute stream of the first plan, so a call can be
- * captured in a CUDA graph (after one call with the same field counts, which
- * allocates the work buffers and the work list).  Plans in a group get a
+ * All launches are ordered by the compute stream of the first plan, so a call
+ * can be captured in a CUDA graph (after one call with the same field counts,
+ * which allocates the work buffers and the work list).  Plans in a group get a
  * common checkpoint spacing.  No counterpart in SHTns 3.5.2. */
 typedef struct shtns_b200_group* shtns_group;
 shtns_group shtns_b200_group_create(int nplans, shtns_cfg* plans);
