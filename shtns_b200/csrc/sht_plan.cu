@@ -566,13 +566,17 @@ extern "C" int shtns_set_grid_auto(shtns_cfg s, enum shtns_type flags, double ep
 	// 13.2 GB; 25.5 and 24.7 ms against 28.6 and 26.1 ms at 32 for the Legendre
 	// stages of 8 fields, whose tiles are generated in chains of one segment),
 	// else every 32
-	size_t mem_free = 0, mem_total = 0;
-	if (cudaMemGetInfo(&mem_free, &mem_total) != cudaSuccess) { cudaGetLastError(); mem_total = 0; }
 	for (s->ckseg = 8; s->ckseg < LG_SEG; s->ckseg *= 2) {
 		long segs = 0;
 		for (int im = 0; im <= s->mmax; im++) segs += (s->kmax_h[im] + s->ckseg - 1) / s->ckseg;
 		const double bytes = (double) segs * s->nlat_2 * 16.0;
-		if (bytes <= (s->ckseg == 8 ? 512.0 * 1024 * 1024 : std::min(16.0 * 1024 * 1024 * 1024, 0.125 * mem_total))) break;
+		double limit = 512.0 * 1024 * 1024;
+		if (s->ckseg > 8) {
+			size_t mem_free = 0, mem_total = 0;
+			if (cudaMemGetInfo(&mem_free, &mem_total) != cudaSuccess) { cudaGetLastError(); mem_total = 0; }
+			limit = std::min(16.0 * 1024 * 1024 * 1024, 0.125 * mem_total);
+		}
+		if (bytes <= limit) break;
 	}
 	checkpoint_offsets(s);
 	if (init_device(s) != 0) { plan_error("GPU initialisation failed: " + g_last_error); return -1; }
