@@ -444,16 +444,29 @@ void launch_checkpoints(shtns_cfg s, cudaStream_t st)
 	cudaFree(d_nseg);
 }
 
-// Fields per CTA of the prologue and epilogue kernels: 1
-// or 2 for so many, else the largest of 16, 8 and 4 that leaves the fewest
-// idle (fewer than 4 split the 64-byte groups of four field-components)
-static int tile_fields(int n)
+// Fields per CTA of the prologue and epilogue kernels: 1 or 2 for so many, else
+// 16, 8 or 4 (fewer split the 64-byte groups of four field-components),
+// whichever leaves the fewest items idle: the fields round up to the tile, and
+// the rows of an order by half a tile of rows(f) on average.  (By the fields
+// alone 156 vector fields took 4 at a time and 128 rows, of which lmax 63 has
+// 33: prologue 22 us, epilogue 20; here 17 and 15.)
+template <class Rows>
+static int tile_fields(int n, int mean_rows, Rows rows)
 {
 	if (n <= 2) return n;
-	int best = 16;
-	for (int f = 8; f >= 4; f /= 2)
-		if ((n + f - 1) / f * f < (n + best - 1) / best * best) best = f;
+	int best = 0;
+	long least = 0;
+	for (int f = 16; f >= 4; f /= 2) {
+		const long items = (long) ((n + f - 1) / f * f) * (2 * mean_rows + rows(f));
+		if (!best || items < least) { best = f; least = items; }
+	}
 	return best;
+}
+
+// Ishioka rows of an order on average, up to degree lmax
+static int mean_rows(const PrepParams& p, int lmax, int mmax)
+{
+	return (2 * (lmax + 1) - (p.im0 + mmax) * p.mres) / 4 + 1;
 }
 
 void launch_prep_synth(const PrepParams& p, cudaStream_t st)
@@ -465,10 +478,11 @@ void launch_prep_synth(const PrepParams& p, cudaStream_t st)
 		dim3 grid((kmax0 + K - 1) / K, (p.nf + PF - 1) / PF * ngroups, p.mlim + 1 - p.im0);
 		kern<<<grid, 256, 0, st>>>(p);
 	};
+	const int pf = tile_fields(p.nf, mean_rows(p, p.llim, p.mlim), [](int f) { return pt_items(f) / f; });
 	auto pick = [&](auto c, auto VC) {
 		using C = decltype(c);
 		constexpr bool V = decltype(VC)::value;
-		switch (tile_fields(p.nf)) {
+		switch (pf) {
 			case 1: go(prep_synth_kernel<1, C, V>, 1); break;
 			case 2: go(prep_synth_kernel<2, C, V>, 2); break;
 			case 4: go(prep_synth_kernel<4, C, V>, 4); break;
@@ -585,9 +599,10 @@ void launch_post_analys_m(const PrepParams& p, int mmax, cudaStream_t st)
 		dim3 grid((p.lmax + J) / J, (p.nf + PF - 1) / PF * ngroups, mmax + 1 - p.im0);
 		kern<<<grid, 256, 0, st>>>(p);
 	};
+	const int pf = tile_fields(p.nf, mean_rows(p, p.lmax, mmax), [](int f) { return f == 16 ? PostTile<16>::J / 2 : f == 8 ? PostTile<8>::J / 2 : PostTile<4>::J / 2; });
 	auto pick = [&](auto c) {
 		using C = decltype(c);
-		switch (tile_fields(p.nf)) {
+		switch (pf) {
 			case 1: go(post_analys_kernel<1, C>, 1, PostTile<1>::J); break;
 			case 2: case 4: go(post_analys_kernel<4, C>, 4, PostTile<4>::J); break;
 			case 8: go(post_analys_kernel<8, C>, 8, PostTile<8>::J); break;
