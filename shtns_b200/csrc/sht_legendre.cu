@@ -445,28 +445,27 @@ void launch_checkpoints(shtns_cfg s, cudaStream_t st)
 }
 
 // Fields per CTA of the prologue and epilogue kernels: 1 or 2 for so many, else
-// 16, 8 or 4 (fewer split the 64-byte groups of four field-components),
-// whichever leaves the fewest items idle: the fields round up to the tile, and
-// the rows of an order by half a tile of rows(f) on average.  (By the fields
-// alone 156 vector fields took 4 at a time and 128 rows, of which lmax 63 has
-// 33: prologue 22 us, epilogue 20; here 17 and 15.)
+// 16, 8 or 4 (fewer split the 64-byte groups of four field-components).  A call
+// whose CTAs of 4 fields are at most two per SM takes those: the less a CTA has
+// to do the sooner the call ends (12 vector fields at lmax 63: prologue 9.0
+// and epilogue 8.7 us, with 16 fields a CTA 12.0 and 10.6).  Beyond, whichever
+// leaves the fewest items idle: the fields round up to the tile, and the rows of an order by half a
+// tile of rows(f) on average.  (By the fields alone 156 vector fields took 4 at
+// a time and 128 rows, of which lmax 63 has 33: 22 / 20 us, here 17 / 15.)
 template <class Rows>
-static int tile_fields(int n, int mean_rows, Rows rows)
+static int tile_fields(const PrepParams& p, int lmax, int mmax, int groups, Rows rows)
 {
-	if (n <= 2) return n;
+	if (p.nf <= 2) return p.nf;
+	const int rows2 = lmax + 3 - (p.im0 + mmax) * p.mres / 2;     // twice the mean rows of an order
+	const long ctas4 = (long) ((p.nf + 3) / 4) * groups * (mmax + 1 - p.im0) * (((lmax - p.im0 * p.mres) / 2 + rows(4)) / rows(4));
+	if (ctas4 <= 2 * 148) return 4;
 	int best = 0;
 	long least = 0;
 	for (int f = 16; f >= 4; f /= 2) {
-		const long items = (long) ((n + f - 1) / f * f) * (2 * mean_rows + rows(f));
+		const long items = (long) ((p.nf + f - 1) / f * f) * (rows2 + rows(f));
 		if (!best || items < least) { best = f; least = items; }
 	}
 	return best;
-}
-
-// Ishioka rows of an order on average, up to degree lmax
-static int mean_rows(const PrepParams& p, int lmax, int mmax)
-{
-	return (2 * (lmax + 1) - (p.im0 + mmax) * p.mres) / 4 + 1;
 }
 
 void launch_prep_synth(const PrepParams& p, cudaStream_t st)
@@ -478,7 +477,7 @@ void launch_prep_synth(const PrepParams& p, cudaStream_t st)
 		dim3 grid((kmax0 + K - 1) / K, (p.nf + PF - 1) / PF * ngroups, p.mlim + 1 - p.im0);
 		kern<<<grid, 256, 0, st>>>(p);
 	};
-	const int pf = tile_fields(p.nf, mean_rows(p, p.llim, p.mlim), [](int f) { return pt_items(f) / f; });
+	const int pf = tile_fields(p, p.llim, p.mlim, ngroups, [](int f) { return pt_items(f) / f; });
 	auto pick = [&](auto c, auto VC) {
 		using C = decltype(c);
 		constexpr bool V = decltype(VC)::value;
@@ -599,7 +598,7 @@ void launch_post_analys_m(const PrepParams& p, int mmax, cudaStream_t st)
 		dim3 grid((p.lmax + J) / J, (p.nf + PF - 1) / PF * ngroups, mmax + 1 - p.im0);
 		kern<<<grid, 256, 0, st>>>(p);
 	};
-	const int pf = tile_fields(p.nf, mean_rows(p, p.lmax, mmax), [](int f) { return f == 16 ? PostTile<16>::J / 2 : f == 8 ? PostTile<8>::J / 2 : PostTile<4>::J / 2; });
+	const int pf = tile_fields(p, p.lmax, mmax, ngroups, [](int f) { return f == 16 ? PostTile<16>::J / 2 : f == 8 ? PostTile<8>::J / 2 : PostTile<4>::J / 2; });
 	auto pick = [&](auto c) {
 		using C = decltype(c);
 		switch (pf) {
