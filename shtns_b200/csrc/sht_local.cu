@@ -316,8 +316,8 @@ struct PtsState {
 template <int NC, bool GATE>
 __device__ __forceinline__ void pts_add(PtsState<NC>& z, double2 q, double2 s, double2 t)
 {
-	double y = z.y1, d = z.d1;
-	if (GATE && z.E) { y = 0.0; d = 0.0; }
+	const double y = z.y1, d = z.d1;
+	if (GATE && z.E) q = s = t = make_double2(0.0, 0.0);      // not y = 0: an infinite coefficient would make a NaN
 	z.q = cfma(y, q, z.q);
 	if constexpr (NC == 3) {
 		z.sdt = cfma(d, s, z.sdt); z.sy = cfma(y, s, z.sy);
@@ -365,6 +365,7 @@ __global__ void __launch_bounds__(512) points_kernel(LocalParams p, const double
 		PtsState<NC> z[P];
 		double s2[P];
 		const int n = p.ltr - m;              // degrees beyond m
+		unsigned dead = 0;                    // points (bit u) that this order leaves out
 		// bits by which the values can grow over the n steps: while they grow,
 		// P_l <= a_l P_{l-1} (b_l < 0 only takes away), a_l <= 2 sqrt(ltr / (l - m)),
 		// so by at most sqrt((4 ltr)^n / n!), and n! >= (n / e)^n
@@ -384,7 +385,7 @@ __global__ void __launch_bounds__(512) points_kernel(LocalParams p, const double
 			}
 			y *= cm;
 			if (E >= -LOC_FOLD) { y = ldexp(y, E); E = 0; }
-			else if ((float) E + grow < -200.0f) { y = 0.0; E = 0; }      // no degree kept of this order can matter here
+			else if ((float) E + grow < -200.0f) { y = 0.0; E = 0; dead |= 1u << u; }      // no degree kept of this order can matter here
 			z[u].E = E;
 			z[u].y0 = 0.0; z[u].y1 = y;
 			z[u].d0 = 0.0; z[u].d1 = (m > 0) ? x[u] * m * y : 0.0;
@@ -463,6 +464,7 @@ __global__ void __launch_bounds__(512) points_kernel(LocalParams p, const double
 		}
 		#pragma unroll
 		for (int u = 0; u < P; u++) {
+			if (dead >> u & 1) z[u].q = z[u].sdt = z[u].tdt = z[u].sy = z[u].ty = zero;      // (with an infinite coefficient: NaNs)
 			const double c2 = im ? 2.0 : 1.0, sr = (m > 0) ? st[u] : 1.0;
 			const double C = c2 * cs[u], D = c2 * sn[u];
 			v[u][0] += (z[u].q.x * sr) * C - (m > 0 ? (z[u].q.y * sr) * D : 0.0);

@@ -244,3 +244,35 @@ def test_many_points_equal_the_kernel_per_point(lmax, mmax, mres, npts):
         a, b = vec(c, p, S), vec(c[pick].contiguous(), p[pick].contiguous(), S)
         for x, y in zip(a, b):
             assert np.abs(x[pick] - y).max() <= tol * max(np.abs(x).max(), 1e-300)
+
+
+def test_orders_left_out_ignore_infinite_coefficients():
+    """Orders whose Legendre functions are below 2^-600 at a point are left out
+    of its sums, by the kernels for many points as by the kernel per point: an
+    infinite or undefined coefficient there does not reach the value.  lmax 2047:
+    at sin(theta) 0.35 degree 1000 of order 1000 starts at 2^-1500 and the order
+    counts from a later degree on; order 2000 never does; at the equator both do."""
+    import torch
+    import shtns_b200
+    dev = torch.device("cuda:0")
+    lmax = 2047
+    sh = shtns_b200.sht(lmax)
+    polar = np.repeat([True, False], 150)
+    ct = torch.from_numpy(np.where(polar, np.linspace(0.936, 0.94, 300), np.linspace(0.0, 0.05, 300))).to(dev)
+    ph = torch.linspace(0.0, 6.0, 300, dtype=torch.float64, device=dev)
+    sh._stream()
+
+    def vec(Q, S, T, n):
+        out = [torch.empty(n, dtype=torch.float64, device=dev) for _ in range(3)]
+        sh._lib.shtns_b200_SHqst_to_points(sh._cfg, *[C.c_void_p(x.data_ptr()) for x in (Q, S, T, ct, ph)], *[C.c_void_p(o.data_ptr()) for o in out], n)
+        return torch.stack(out).cpu().numpy()
+    clean = torch.from_numpy(rand_spec(lmax, lmax, 1, 90)).to(dev)
+    for m, bad in ((1000, np.inf), (2000, np.inf), (2000, np.nan)):
+        q = clean.clone()
+        q[int(sh.idx(m, m))] = bad
+        v, few = sh.points(q, ct, ph).cpu().numpy(), sh.points(q, ct[:100].contiguous(), ph[:100].contiguous()).cpu().numpy()
+        assert np.isfinite(few).all() and np.array_equal(np.isfinite(v), polar)
+        assert np.abs(v[:100] - few).max() <= 4 * lmax * 2.0 ** -53 * 6.0 * np.abs(few).max()
+        for c in range(3):
+            x = vec(*[q if i == c else clean for i in range(3)], 300)
+            assert np.isfinite(x[:, polar]).all() and not np.isfinite(x[:, ~polar]).all()
