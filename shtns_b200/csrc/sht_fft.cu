@@ -234,14 +234,14 @@ __device__ __forceinline__ void fused_fft(double2* X, const double2* tw, int sig
 	// first pass: butterfly b reads elements b + q*N/R0 from global, no twiddles
 	using G = Geo<N, S>;
 	constexpr int NBF = N / R0, TOT = S * NBF, NB = (TOT + G::T - 1) / G::T;
-	double2 u[NB][R0];
+	decltype(ld(0, 0)) in[NB][R0];
 	#pragma unroll
 	for (int i = 0; i < NB; i++) {
 		const int g = tid + i * G::T;
 		if (g < TOT) {
 			const int s = g % S, b = g / S;
 			#pragma unroll
-			for (int q = 0; q < R0; q++) u[i][q] = ld(s, b + q * NBF);
+			for (int q = 0; q < R0; q++) in[i][q] = ld(s, b + q * NBF);
 		}
 	}
 	#pragma unroll
@@ -249,9 +249,12 @@ __device__ __forceinline__ void fused_fft(double2* X, const double2* tw, int sig
 		const int g = tid + i * G::T;
 		if (g < TOT) {
 			const int s = g % S, b = g / S;
-			Dft<R0>::run(u[i], sign);
+			double2 u[R0];
 			#pragma unroll
-			for (int q = 0; q < R0; q++) X[G::at(s, b * R0 + q)] = u[i][q];
+			for (int q = 0; q < R0; q++) u[q] = widen(in[i][q]);
+			Dft<R0>::run(u, sign);
+			#pragma unroll
+			for (int q = 0; q < R0; q++) X[G::at(s, b * R0 + q)] = u[q];
 		}
 	}
 	__syncthreads();
@@ -301,11 +304,13 @@ __global__ void __launch_bounds__(Geo<N, S>::T) fft3_analys_kernel(FftParams p)
 	const int c = fc / p.nf;
 	const G* in = grid_in<G>(p, c, fc);
 	const bool phi = p.phi_contiguous, v2 = p.vec2;
-	auto ld = [&](int s, int j) -> double2 {
+	auto ld = [&](int s, int j) {
 		const int row = lat0 + 2 * s;
-		if (row >= nlat) return make_double2(0.0, 0.0);
+		typename Pair<G>::T v = {};
+		if (row >= nlat) return v;
 		if (!phi) return load_pair(in + (long)j * nlat + row, v2);
-		return make_double2(__ldg(in + (long)row * N + j), __ldg(in + (long)(row + 1) * N + j));
+		v.x = __ldg(in + (long)row * N + j); v.y = __ldg(in + (long)(row + 1) * N + j);
+		return v;
 	};
 	// Fourier rows straight from the last radix pass (pairs z_k, z_{N-k})
 	double2* Ff = p.F + (long)fc * p.fstride;
@@ -649,10 +654,7 @@ __global__ void __launch_bounds__(Geo<N, S>::T, fft4_minb(S * N)) fft4_analys_ke
 		const int lat0 = (tile - fc * tt.nlg) * 2 * S;
 		int rs = 2 * S;                         // opaque per tile, as mlim in the synthesis
 		asm volatile("" : "+r"(rs));
-		auto ld = [&](int s, int j) -> double2 {
-			const typename Pair<G>::T v = *reinterpret_cast<const typename Pair<G>::T*>(stg + j * rs + 2 * s);
-			return make_double2(v.x, v.y);
-		};
+		auto ld = [&](int s, int j) { return *reinterpret_cast<const typename Pair<G>::T*>(stg + j * rs + 2 * s); };
 		const int next = tile + gridDim.x;
 		auto prefetch = [&]() {
 			if (threadIdx.x == 0 && next < tt.ntiles) {

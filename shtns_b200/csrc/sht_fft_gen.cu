@@ -69,8 +69,11 @@ __device__ int g_gen_wait_err;                   // set when a bounded wait gave
 __device__ __forceinline__ void opaque(int& v) { asm volatile("" : "+r"(v)); }
 
 // input element j of the sequence, from the staged tile (STG) or global memory
+// (of the analysis as it is stored: see load_pair)
+template <bool SYNTH, class G> using GenIn = std::conditional_t<SYNTH, double2, typename Pair<G>::T>;
+
 template <bool SYNTH, bool STG, bool PHI, class G>
-__device__ __forceinline__ double2 gen_load(const GenTile<G>& t, int j)
+__device__ __forceinline__ GenIn<SYNTH, G> gen_load(const GenTile<G>& t, int j)
 {
 	if constexpr (SYNTH) {
 		// Z_j = A_j + i B_j (j <= ml), Z_{N-j} = conj(A_j) + i conj(B_j), zero between
@@ -93,13 +96,14 @@ __device__ __forceinline__ double2 gen_load(const GenTile<G>& t, int j)
 		if (k == 0) { a.y = 0.0; b.y = 0.0; }
 		return lo ? make_double2(a.x - b.y, a.y + b.x) : make_double2(a.x + b.y, b.x - a.y);
 	} else if constexpr (STG) {
-		const typename Pair<G>::T v = static_cast<const typename Pair<G>::T*>(t.stg)[j * t.S];
-		return make_double2(v.x, v.y);
-	} else if constexpr (PHI) {
-		const G* i0 = t.in + (long)t.row * t.N + j;
-		return t.live ? make_double2(__ldg(i0), __ldg(i0 + t.N)) : make_double2(0.0, 0.0);
+		return static_cast<const typename Pair<G>::T*>(t.stg)[j * t.S];
 	} else {
-		return t.live ? load_pair(t.in + (long)j * t.nlat + t.row, t.v2) : make_double2(0.0, 0.0);
+		typename Pair<G>::T v = {};
+		if constexpr (PHI) {
+			const G* i0 = t.in + (long)t.row * t.N + j;
+			if (t.live) { v.x = __ldg(i0); v.y = __ldg(i0 + t.N); }
+		} else if (t.live) v = load_pair(t.in + (long)j * t.nlat + t.row, t.v2);
+		return v;
 	}
 }
 
@@ -110,13 +114,13 @@ __device__ __forceinline__ void gen_first(GenTile<G> t, int nbf)
 {
 	opaque(t.b0);
 	constexpr int NB = E / R;
-	double2 u[NB][R];
+	GenIn<SYNTH, G> in[NB][R];
 	#pragma unroll
 	for (int i = 0; i < NB; i++) {
 		const int b = t.b0 + i * t.bstep;
 		if (b < nbf) {
 			#pragma unroll
-			for (int q = 0; q < R; q++) u[i][q] = gen_load<SYNTH, STG, PHI>(t, b + q * nbf);
+			for (int q = 0; q < R; q++) in[i][q] = gen_load<SYNTH, STG, PHI>(t, b + q * nbf);
 		}
 	}
 	if constexpr (STG) __syncthreads();
@@ -124,9 +128,12 @@ __device__ __forceinline__ void gen_first(GenTile<G> t, int nbf)
 	for (int i = 0; i < NB; i++) {
 		const int b = t.b0 + i * t.bstep;
 		if (b < nbf) {
-			Dft<R>::run(u[i], SYNTH ? 1 : -1);
+			double2 u[R];
 			#pragma unroll
-			for (int q = 0; q < R; q++) t.Xs[pos(b * R + q)] = u[i][q];
+			for (int q = 0; q < R; q++) u[q] = widen(in[i][q]);
+			Dft<R>::run(u, SYNTH ? 1 : -1);
+			#pragma unroll
+			for (int q = 0; q < R; q++) t.Xs[pos(b * R + q)] = u[q];
 		}
 	}
 	__syncthreads();

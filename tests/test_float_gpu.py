@@ -13,7 +13,8 @@ from tests.common import rand_spec
 pytestmark = pytest.mark.gpu
 
 GRIDS = [(127, 192, 384, "theta"), (127, 190, 384, "theta"), (127, 192, 384, "phi"), (63, 66, 128, "theta"), (63, 66, 128, "phi"), (40, 42, 125, "theta"),
-         (255, 384, 768, "theta"), (511, 514, 1536, "theta"), (63, 64, 6144, "theta"), (31, 34, 3072, "theta")]
+         (255, 384, 768, "theta"), (511, 514, 1536, "theta"), (63, 64, 6144, "theta"), (31, 34, 3072, "theta"), (40, 128, 360, "theta"), (40, 130, 360, "theta"), (40, 128, 360, "phi"), (40, 128, 4096, "theta"),
+         (40, 128, 4096, "phi"), (63, 66, 192, "phi"), (63, 66, 768, "phi"), (63, 66, 1536, "theta"), (63, 64, 1536, "phi")]
 
 
 @pytest.mark.parametrize("lmax,nlat,nphi,layout", GRIDS)
