@@ -190,7 +190,7 @@ void run_analys(shtns_cfg s, int ncomp, const int* types, const double* i0, cons
 	fp.spat_in[0] = i0; fp.spat_in[1] = i1; fp.spat_in[2] = i2;
 	fp.f32 = f32;
 	fp.vec2 = aligned16(i0, i1, i2, s->spat_dist, f32);
-	if (s->d_tw4 && !s->phi_contiguous && fp.vec2 && s->fft_generic == 0) {
+	if (fft_fourstep_used(fp, j.nfc, false)) {
 		// the four-step FFT analysis needs a grid per field-component of scratch
 		// (without room for it, or where a stream capture forbids the allocation,
 		// the direct kernels run instead)

@@ -817,16 +817,10 @@ bool launch_fft4_n(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 	}
 }
 
-// four-step path on theta-contiguous grids with 16-byte aligned latitude pairs
-// and (analysis) a scratch grid; false otherwise.  Against the one-pass kernels,
-// synthesis / analysis: nphi 6144, 8 grids of 3072 latitudes 1552/1155 ->
-// 866/803 us; the synthesis of nphi 3072, 32 grids of 1536 latitudes 1417 -> 783
-// us (its one-pass kernel stores 16 bytes of each grid row, half a sector).
-template <int N1, int N2>
-bool launch_fourstep(const FftParams& p, int nfc, cudaStream_t st, bool synth)
+// Four-step kernels, for a call that fft_fourstep_used admits.
+template <int N1, int N2, bool ANALYS = true>
+void launch_fourstep(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 {
-	if (p.N != N1 * N2 || p.phi_contiguous || !p.vec2 || !p.tw1 || p.generic != 0 || p.f32 || (!synth && !p.scratch)) return false;
-	if (p.nlat % 2 || ((uintptr_t) p.F & 31)) return false;
 	using G1 = Geo<N1, FS_S>;
 	using G2 = Geo<N2, FS_S>;
 	using G3 = Geo<N1, 2 * FS_S>;
@@ -836,12 +830,11 @@ bool launch_fourstep(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 	if (synth) {
 		fft_fs_synth1_kernel<N1, N2><<<dim3(nlb, N2, nfc), G1::T, s1, st>>>(p);
 		fft_fs_synth2_kernel<N1, N2><<<dim3(nlb, N1, nfc), G2::T, s2, st>>>(p);
-	} else {
+	} else if constexpr (ANALYS) {
 		fft_fs_analys1_kernel<N1, N2><<<dim3(nlb, N1, nfc), G2::T, s2, st>>>(p);
 		fft_fs_analys2_kernel<N1, N2><<<dim3(nlb, N2 / 2 + 1, nfc), G3::T, s3, st>>>(p);
 	}
 	shtb_count_launch();         // the second of the two launches is counted by the caller
-	return true;
 }
 
 template <int N1, int N2>
@@ -853,11 +846,14 @@ void set_fourstep_limits()
 
 bool launch_fused(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 {
-	if (launch_fourstep<96, 128>(p, nfc, st, synth) || launch_fourstep<64, 96>(p, nfc, st, synth)) return true;
-	// nphi 3072: the synthesis of grids that do not stay in the L2 cache, where
-	// the half sectors of the one-pass kernel would be completed (3 grids of 1536
-	// latitudes: 100 -> 83 us)
-	if (synth && (size_t) nfc * p.N * p.nlat * 8 > ((size_t) 96 << 20) && launch_fourstep<48, 64>(p, nfc, st, synth)) return true;
+	if (fft_fourstep_used(p, nfc, synth) && (synth || p.scratch)) {
+		switch (p.N) {
+			case 12288: launch_fourstep<96, 128>(p, nfc, st, synth); break;
+			case 6144: launch_fourstep<64, 96>(p, nfc, st, synth); break;
+			default: launch_fourstep<48, 64, false>(p, nfc, st, synth); break;      // 3072: synthesis only
+		}
+		return true;
+	}
 	if (p.generic == 0 || p.generic == 3) {
 		bool done = false;
 		switch (p.N) {
@@ -966,6 +962,22 @@ void launch_fft_analys(const FftParams& p, int nfc, cudaStream_t st)
 	g_last_fft_path = 0;
 	launch_fft_gen(p, nfc, st, false);
 	shtb_count_launch();
+}
+
+// Whether a call takes the four-step kernels (the analysis then needs a grid
+// per field-component in p.scratch): FP64, theta-contiguous grids with 16-byte
+// aligned latitude pairs; nphi 6144 and 12288, and the synthesis of nphi 3072
+// where the grids do not stay in the L2 cache, in which the half sectors that
+// the one-pass kernel stores would be completed.  Against the one-pass kernels,
+// synthesis / analysis: nphi 6144, 8 grids of 3072 latitudes 1552/1155 ->
+// 866/803 us; the synthesis of nphi 3072, 32 grids of 1536 latitudes 1417 -> 783,
+// 3 grids 100 -> 83 us.  The launcher, the allocation of the scratch and the
+// single-precision entry points all ask here.
+bool fft_fourstep_used(const FftParams& p, int nfc, bool synth)
+{
+	if (p.phi_contiguous || !p.vec2 || !p.tw1 || p.generic != 0 || p.f32 || p.nlat % 2 || ((uintptr_t) p.F & 31)) return false;
+	if (p.N == 3072) return synth && (size_t) nfc * p.N * p.nlat * 8 > ((size_t) 96 << 20);
+	return p.N == 6144 || p.N == 12288;
 }
 
 // nphi = n1 n2 of the four-step kernels

@@ -284,6 +284,7 @@ void launch_leg_multi(const LegParams* d_plist, const int4* d_work, int nwork, i
                       int nctas, cudaStream_t st);
 bool fft_fused_available(int N);
 bool fft_fourstep_factors(int N, int& n1, int& n2);
+bool fft_fourstep_used(const FftParams& p, int nfc, bool synth);
 size_t fft_smem_bytes(int N, int S);
 bool fft_gen_plan(int N, FftGenPlan& g, int emax);
 void launch_fft_gen(const FftParams& p, int nfc, cudaStream_t st, bool synth);

@@ -74,3 +74,25 @@ def test_float_arrays_at_odd_addresses():
         lib.cu_spat_to_SH_float(sh._cfg, C.c_void_p(want.data_ptr()), C.c_void_p(ref.data_ptr()), 63)
         assert torch.equal(back[1:], torch.view_as_real(ref).flatten()) and float(back[0]) == 0.0
         assert lib.shtns_b200_status() == 0
+
+
+@pytest.mark.parametrize("nphi,layout,fourstep", [(3072, "theta", False), (3072, "phi", False), (6144, "phi", False), (6144, "theta", True)])
+def test_device_memory_of_four_step_lengths(nphi, layout, fourstep):
+    """Only a call that takes the four-step kernels pays for them: the analysis
+    with a scratch grid per field.  Here: the theta-contiguous 6144 (3072 has a four-step synthesis only,
+    for grids beyond 96 MB)."""
+    import shtns_b200
+    from shtns_b200 import capi
+    lib = capi.load()
+    dev = torch.device("cuda:0")
+    sh = shtns_b200.sht(31)
+    sh.set_grid(34, nphi, flags=shtns_b200.sht_quick_init | (shtns_b200.SHT_THETA_CONTIGUOUS if layout == "theta" else shtns_b200.SHT_PHI_CONTIGUOUS),
+                polar_opt=1e-10)
+    nf = 8
+    grids = 8 * nf * sh.nspat
+    q = torch.from_numpy(rand_spec(31, 31, 1, 5, nfields=nf)).to(dev)
+    v = sh.synth(q)
+    before = lib.shtns_b200_device_bytes(sh._cfg)
+    sh.analys(v)
+    after = lib.shtns_b200_device_bytes(sh._cfg)
+    assert after - before == (grids if fourstep else 0)
