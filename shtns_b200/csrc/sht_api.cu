@@ -452,8 +452,8 @@ extern "C" void cu_spat_to_SH_adjoint(shtns_cfg s, cplx* Qg, double* Vg, int ltr
 // the FFT kernels convert the grid at their edges: no FP64 copy of either.
 // Measured: 128 fields at lmax 255 through the autograd functions (four transforms and
 // the user's products) 2.10 -> 1.45 ms.
-// The four-step FFT (nphi 6144 and 12288) has no float form (its synthesis keeps an
-// intermediate in the output grid): those plans convert through the staging
+// The four-step FFT has no float form (its synthesis keeps an intermediate in
+// the output grid): calls that it would serve convert through the staging
 // buffer, and so do calls whose coefficients are not aligned to 8 bytes.
 namespace {
 __global__ void f2d_kernel(const float* __restrict__ in, double* __restrict__ out, long n)
@@ -475,10 +475,21 @@ void convert(const double* in, float* out, long n, cudaStream_t st)
 	shtb_count_launch();
 }
 
+// float arrays that go through the staging buffer
+bool float_staged(shtns_cfg s, const cplx_f* Qlm, int ltr, bool synth)
+{
+	if ((uintptr_t) Qlm & 7) return true;
+	Job j;
+	if (!s->d_tw4 || !setup_job(s, j, 1, T_SCAL, ltr, 0)) return false;
+	FftParams fp = fft_params(s, j);
+	fp.vec2 = s->spat_dist % 2 == 0;                    // of the staged grid
+	return fft_fourstep_used(fp, j.nfc, synth);
+}
+
 void synth_float(shtns_cfg s, const cplx_f* Qlm, float* Vr, int ltr, int adjoint)
 {
 	if (!s || !s->grid_set) { shtb_set_error(1, "transform on a plan without grid"); return; }
-	if (!s->d_tw4 && !((uintptr_t) Qlm & 7)) {
+	if (!float_staged(s, Qlm, ltr, true)) {
 		run_synth(s, 1, T_SCAL, reinterpret_cast<const cplx*>(Qlm), nullptr, nullptr, reinterpret_cast<double*>(Vr), nullptr, nullptr, ltr,
 		          adjoint, 1);
 		return;
@@ -496,7 +507,7 @@ void synth_float(shtns_cfg s, const cplx_f* Qlm, float* Vr, int ltr, int adjoint
 void analys_float(shtns_cfg s, const float* Vr, cplx_f* Qlm, int ltr, int adjoint)
 {
 	if (!s || !s->grid_set) { shtb_set_error(1, "transform on a plan without grid"); return; }
-	if (!s->d_tw4 && !((uintptr_t) Qlm & 7)) {
+	if (!float_staged(s, Qlm, ltr, false)) {
 		run_analys(s, 1, T_SCAL, reinterpret_cast<const double*>(Vr), nullptr, nullptr, reinterpret_cast<cplx*>(Qlm), nullptr, nullptr, ltr,
 		           adjoint, 1);
 		return;

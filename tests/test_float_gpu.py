@@ -13,7 +13,8 @@ from tests.common import rand_spec
 pytestmark = pytest.mark.gpu
 
 GRIDS = [(127, 192, 384, "theta"), (127, 190, 384, "theta"), (127, 192, 384, "phi"), (63, 66, 128, "theta"), (63, 66, 128, "phi"), (40, 42, 125, "theta"),
-         (255, 384, 768, "theta"), (511, 514, 1536, "theta"), (63, 64, 6144, "theta"), (31, 34, 3072, "theta"), (40, 128, 360, "theta"), (40, 130, 360, "theta"), (40, 128, 360, "phi"), (40, 128, 4096, "theta"),
+         (255, 384, 768, "theta"), (511, 514, 1536, "theta"), (63, 64, 6144, "theta"), (63, 64, 6144, "phi"), (31, 34, 12288, "phi"), (31, 34, 3072, "theta"), (31, 36, 3072, "phi"),
+         (31, 1536, 3072, "theta"), (40, 128, 360, "theta"), (40, 130, 360, "theta"), (40, 128, 360, "phi"), (40, 128, 4096, "theta"),
          (40, 128, 4096, "phi"), (63, 66, 192, "phi"), (63, 66, 768, "phi"), (63, 66, 1536, "theta"), (63, 64, 1536, "phi")]
 
 
@@ -79,10 +80,11 @@ def test_float_arrays_at_odd_addresses():
 @pytest.mark.parametrize("nphi,layout,fourstep", [(3072, "theta", False), (3072, "phi", False), (6144, "phi", False), (6144, "theta", True)])
 def test_device_memory_of_four_step_lengths(nphi, layout, fourstep):
     """Only a call that takes the four-step kernels pays for them: the analysis
-    with a scratch grid per field.  Here: the theta-contiguous 6144 (3072 has a four-step synthesis only,
+    with a scratch grid per field, the FP32 transforms with FP64 copies of their
+    arrays.  Here: the theta-contiguous 6144 (3072 has a four-step synthesis only,
     for grids beyond 96 MB)."""
     import shtns_b200
-    from shtns_b200 import capi
+    from shtns_b200 import autograd, capi
     lib = capi.load()
     dev = torch.device("cuda:0")
     sh = shtns_b200.sht(31)
@@ -96,3 +98,7 @@ def test_device_memory_of_four_step_lengths(nphi, layout, fourstep):
     sh.analys(v)
     after = lib.shtns_b200_device_bytes(sh._cfg)
     assert after - before == (grids if fourstep else 0)
+    with torch.no_grad():
+        autograd.analys(sh, autograd.synth(sh, q.to(torch.complex64)))
+    staged = lib.shtns_b200_device_bytes(sh._cfg) - after
+    assert staged >= grids if fourstep else staged == 0
