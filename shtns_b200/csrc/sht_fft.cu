@@ -844,8 +844,30 @@ void set_fourstep_limits()
 	                     (int)(sizeof(double2) * 2 * FS_S * Geo<N1, 2 * FS_S>::SEQ));
 }
 
-bool launch_fused(const FftParams& p, int nfc, cudaStream_t st, bool synth)
+// Latitude pairs per CTA of the one-pass kernels where option 1 leaves the
+// choice: what fits the shared memory twice (fft_params), and half of that where
+// the chains of 16 values per thread leave few warps to a CTA and rows of
+// fewer latitudes cost little: phi-contiguous grids, and the FP64 synthesis of
+// nphi 768.  Kernel times, synthesis / analysis, chains before those / with the
+// larger tile / with this one: 51 phi-contiguous grids of 766 x 1536 221/195,
+// 199/203 and 185/169 us; 8 of 384 x 768 13.1/11.1, 14.1/10.1 and 12.2/9.5; 814 of
+// 192 x 384 208/185, 174/159 and 149/145; theta-contiguous synthesis, 8 of 384 x
+// 768 13.4, 14.2 and 13.4, 204 of them 218, 199 and 185.
+int fused_pairs(const FftParams& p, bool synth)
 {
+	if (p.pairs) return p.S;
+	int S = p.S;
+	if (p.phi_contiguous) {
+		if (p.N == 384 || p.N == 768) S = 2;
+		else if (p.N == 1536) S = 1;
+	} else if (synth && p.N == 768 && !p.f32) S = 2;
+	return std::min(S, p.S);
+}
+
+bool launch_fused(const FftParams& p0, int nfc, cudaStream_t st, bool synth)
+{
+	FftParams p = p0;
+	p.S = fused_pairs(p0, synth);
 	if (fft_fourstep_used(p, nfc, synth) && (synth || p.scratch)) {
 		switch (p.N) {
 			case 12288: launch_fourstep<96, 128>(p, nfc, st, synth); break;
