@@ -95,7 +95,9 @@ int shtns_b200_transform(shtns_cfg, cudaStream_t stream, int howmany, int kind, 
  * kernels), 1 = always the generic mixed-radix kernels, 2 = the fused
  * kernels without prefetch, 3 = prefetched loads with per-thread stores.
  * Option 6 (get only): FFT kernels of the last launch in this process, 0
- * generic, 1 fused direct, 2 prefetched.  Option 7 (test hook, default 0):
+ * generic, 1 fused direct, 2 prefetched.  Option 11 (get only): plan of the
+ * last launch of the generic kernels in this process, 100 x (complex values per
+ * thread) + 10 x passes + (1 if the input was staged by tensor copies).  Option 7 (test hook, default 0):
  * bytes, a multiple of 16 up to 4096, that the prefetching FFT kernels wait
  * for beyond what their tensor copies bring; a positive value makes their
  * bounded wait (about one second) give up, so that tests can check the error

@@ -30,6 +30,7 @@
 #include "sht_fft_grid.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <type_traits>
 
@@ -79,9 +80,10 @@ __device__ __forceinline__ GenIn<SYNTH, G> gen_load(const GenTile<G>& t, int j)
 		// Z_j = A_j + i B_j (j <= ml), Z_{N-j} = conj(A_j) + i conj(B_j), zero between
 		const bool lo = j <= t.ml;
 		const int k = lo ? j : t.N - j;
-		if (k > t.ml || (!STG && !t.live)) return make_double2(0.0, 0.0);
+		const bool in = k <= t.ml && (STG || t.live);
 		double2 a, b;
 		if constexpr (STG) {
+			if (!in) return make_double2(0.0, 0.0);
 			// the two latitudes in an order that alternates with the row, so that
 			// the 8 lanes of a shared-memory phase hit distinct banks
 			const int f = (k >> (t.S == 1 ? 2 : (t.S == 2 ? 1 : 0))) & 1;
@@ -90,8 +92,17 @@ __device__ __forceinline__ GenIn<SYNTH, G> gen_load(const GenTile<G>& t, int j)
 			a = f ? u1 : u0;
 			b = f ? u0 : u1;
 		} else {
-			const double2* f = t.Ff + (long)k * t.nlat + t.row;
-			a = __ldg(f); b = __ldg(f + 1);
+			// in the zero band the first element, thrown away: a load on a path
+			// of its own is waited for there.  One 32-byte load for both latitudes
+			// where the rows are aligned.  Kernel times, cold L2, two loads in a
+			// branch / this form: nphi 128, 504 pairs, orders up to nphi / 2
+			// 7.5 / 6.3 us, nphi / 3 6.7 / 6.1; nphi 4096, 64 pairs 19.8 / 16.9 and
+			// 17.5 / 15.5 (with a zero band of nearly all orders the branch would be
+			// 0.1 to 0.3 us faster; both forms in one kernel lose this gain)
+			const double2* f = t.Ff + (in ? (long)k * t.nlat + t.row : 0);
+			if (t.v4) asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y) : "l"(f));
+			else { a = __ldg(f); b = __ldg(f + 1); }
+			if (!in) return make_double2(0.0, 0.0);
 		}
 		if (k == 0) { a.y = 0.0; b.y = 0.0; }
 		return lo ? make_double2(a.x - b.y, a.y + b.x) : make_double2(a.x + b.y, b.x - a.y);
@@ -228,7 +239,7 @@ __device__ __forceinline__ void gen_last(GenTile<G> t, int nbf)
 		default: break; \
 	}
 
-// E: complex values a thread holds (12 or 16); a pass of radix R runs E / R
+// E: complex values a thread holds (8, 12 or 16); a pass of radix R runs E / R
 // butterflies per thread
 // STG: the input tile arrives by tensor copies in the shared buffer that the
 // passes use (box_rows rows per copy, ncopy copies of box_bytes); PHI: direct
@@ -383,16 +394,27 @@ bool fft_gen_plan(int N, FftGenPlan& out, int emax)
 	return true;
 }
 
+static std::atomic<int> g_gen_last{-1};
+
+// The last launch of this file in this process: 100 E + 10 passes + staged.
+int fft_gen_last() { return g_gen_last.load(); }
+
 void launch_fft_gen(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 {
 	// Up to about a wave of latitude pairs the latency of the passes counts, not
 	// the rate: short butterflies (radices <= 8, more threads, less code to
-	// fetch) and direct loads.  nphi 1024, 256 pairs, synthesis / analysis: 16 16 4
-	// staged 23.6/19.0 us, 8 8 4 4 direct 13.1/13.7; nphi 1440, 360 pairs:
-	// 20.8/17.0 and 14.6/14.1; 1440 pairs: 33.2/32.6 and 38.1/33.6.  Plans that
-	// need 16 values per thread lose to one more pass at every size (nphi 1024,
-	// 2560 pairs 41.3/40.9 and 33.2/36.9, 10240 phi-contiguous 87.7/92.1 and
-	// 78.6/92.6), so they stay for the lengths without the other.
+	// fetch) and direct loads.  Kernel times with cold L2, orders up to nphi / 3,
+	// direct / staged: synthesis of 512 pairs at nphi 720 8.2/9.0 us, 1024
+	// 10.2/11.8; analysis 720 8.0/8.5, 1440 13.3/13.1, 2880 32.2/34.4.  The same
+	// synthesis with the longest butterflies the length allows: nphi 256, 256
+	// pairs 5.6 -> 7.6, 1024 9.2 -> 10.5 (with warm caches 4.9 and 6.5).
+	// The synthesis of longer rows is staged all the same (512 pairs, direct /
+	// staged: nphi 1440 17.4/15.4, 2048 23.1/20.1, 4096 59.9/50.1), except up to
+	// 2^19 points, where the whole call is bound by its launches, and with orders
+	// up to less than nphi / 4 (nphi 4096, 192 pairs, nphi / 32: 18.9/20.3 warm).
+	// Plans that need 16 values per thread lose to one more pass in large calls
+	// too (nphi 1024, 2560 pairs 41.3/40.9 and 33.2/36.9, 10240 phi-contiguous
+	// 87.7/92.1 and 78.6/92.6), so they stay for the lengths without the other.
 	const long pairs = (long)((p.nlat + 1) / 2) * nfc;
 	const bool small = pairs <= 1000;
 	const FftGenPlan& g = (p.gen_small->np && (small || p.gen->E == 16)) ? *p.gen_small : *p.gen;
@@ -422,7 +444,8 @@ void launch_fft_gen(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 	// copies can address (phi-contiguous rows are read in whole lines as they are)
 	alignas(64) CUtensorMap maps[3];
 	const int e = p.f32 ? 4 : 8;
-	bool stg = !small && !(p.nlat & 1) && (synth || (p.vec2 && !p.phi_contiguous));
+	const bool long_rows = synth && p.N > 1024 && pairs * p.N > (1 << 19) && 4 * (p.mlim + 1) >= p.N;
+	bool stg = (!small || long_rows) && !(p.nlat & 1) && (synth || (p.vec2 && !p.phi_contiguous));
 	const int rows = synth ? p.mlim + 1 : p.N, row_bytes = synth ? 32 * S : 2 * e * S;
 	const int ncopy = (rows + 255) / 256;
 	const int box = ((rows + ncopy - 1) / ncopy + 15) & ~15;        // a multiple of 16: copies of 128-byte multiples
@@ -437,6 +460,7 @@ void launch_fft_gen(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 	}
 	const size_t sm = std::max(smem(S), (size_t) ncopy * box * row_bytes) + 128;
 	if (sm > 226 * 1024) stg = false;
+	g_gen_last = 100 * g.E + 10 * g.np + (stg ? 1 : 0);
 	auto go = [&](auto kern) {
 		kern<<<grid, T, stg ? sm : smem(S), st>>>(maps[0], maps[1], maps[2], p, g, lgS, seq, ncopy, box, box * row_bytes);
 	};

@@ -39,7 +39,7 @@ struct MTables {
 struct FftPass { int R, P, nbf, ts; float inv_p; };
 struct FftGenPlan {
 	int np = 0;                          // passes (at least 2)
-	int E = 0;                           // complex values a thread holds: 12 or 16
+	int E = 0;                           // complex values a thread holds: 8, 12 or 16
 	FftPass ps[FFT_MAX_PASSES] = {};
 };
 
@@ -290,6 +290,7 @@ bool fft_gen_plan(int N, FftGenPlan& g, int emax);
 void launch_fft_gen(const FftParams& p, int nfc, cudaStream_t st, bool synth);
 void fft_gen_set_smem_limits();
 int fft_gen_take_wait_error();
+int fft_gen_last();
 void launch_fft_synth(const FftParams& p, int nfc, cudaStream_t st);
 void launch_fft_analys(const FftParams& p, int nfc, cudaStream_t st);
 int fft_take_wait_error();

@@ -893,6 +893,7 @@ extern "C" int shtns_b200_get_option(shtns_cfg s, int option)
 		case 4: return s->split_ns;
 		case 5: return s->tile_wm;
 		case 6: return fft_last_path();   // FFT kernels of the last launch in this process
+		case 11: return fft_gen_last();   // plan of the last launch of the generic FFT kernels in this process
 		case 7: return s->fft_extra_tx;
 		case 8: return s->split_form;
 		case 10: return s->ftab_mode;
