@@ -116,6 +116,10 @@ int shtns_b200_transform(shtns_cfg, cudaStream_t stream, int howmany, int kind, 
  * No counterpart in SHTns 3.5.2. */
 int shtns_b200_set_option(shtns_cfg, int option, int value);
 int shtns_b200_get_option(shtns_cfg, int option);
+/* Rule of the checkpoint spacing that set_grid picks: bytes[0 .. 2] = size of
+ * the table at spacings 8, 16 and 32, mem_free = free device memory.  Returns
+ * 8, 16 or 32; set_grid takes the next spacing where the allocation fails. */
+int shtns_b200_checkpoint_spacing(const double* bytes, double mem_free);
 
 /* Option 5 of shtns_b200_set_option: shape of the FP64 Legendre tiles, warps
  * along the rows: 1 = 32 rows x 128 columns, 2 = 64 x 64, 4 = 128 x 32,

@@ -134,6 +134,7 @@ PROTOTYPES = {
     "SHtor_to_spat_ml": (None, [CFG, I, P, P, P, I]),
     "SHqst_to_spat_ml": (None, [CFG, I, P, P, P, P, P, P, I]),
     "spat_to_SHqst_ml": (None, [CFG, I, P, P, P, P, P, P, I]),
+    "shtns_b200_checkpoint_spacing": (I, [P, D]),
     "shtns_b200_kernel_errors": (I, [CFG]),
     "shtns_b200_split_table_bytes": (C.c_size_t, [CFG]),
     "shtns_b200_get_option": (I, [CFG, I]),

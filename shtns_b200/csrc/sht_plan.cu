@@ -319,6 +319,21 @@ static bool nphi_ok(int n)
 	return r == 1 && (fft_smem_bytes(n, 1) <= 227 * 1024 || fft_fused_available(n));
 }
 
+#define CK_SMALL (512.0 * 1024 * 1024)
+
+// Checkpoint spacing for tables of bytes[0 .. 2] at 8, 16 and 32 degree-pairs:
+// 8 or 16 when they take at most 512 MB; 16 also up to 16 GB and a quarter of
+// the free memory (lmax 4095: 13.2 GB; 25.5 and 24.7 ms against 28.6 and 26.1 ms
+// at 32 for the Legendre stages of 8 fields, whose tiles are generated in
+// chains of one segment), the rest being left to the work buffers, the other
+// tables and the caller; else 32.
+extern "C" int shtns_b200_checkpoint_spacing(const double* bytes, double mem_free)
+{
+	if (bytes[0] <= CK_SMALL) return 8;
+	if (bytes[1] <= CK_SMALL) return 16;
+	return bytes[1] <= std::min(16.0 * 1024 * 1024 * 1024, 0.25 * mem_free) ? 16 : 32;
+}
+
 // first checkpoint segment of every order for the current spacing s->ckseg
 static void checkpoint_offsets(shtns_cfg s)
 {
@@ -389,6 +404,21 @@ static int init_device(shtns_cfg s)
 	size_t o = 0;
 	auto put = [&](const std::vector<double>& v) { memcpy(c.data() + o, v.data(), sizeof(double) * v.size()); o += v.size(); };
 	put(s->ish_c); put(s->ish_xs); put(s->ish_xa); put(s->stdt_lo); put(s->stdt_hi); put(s->van_lo); put(s->van_hi); put(s->l_2);
+	// the checkpoint table, at the next spacings when the memory is short
+	bool ok = true;
+	size_t ck_elems;
+	for (;;) {
+		ck_elems = (size_t) s->segtot * n2;
+		const cudaError_t e = cudaMalloc(&s->d_ck, sizeof(double2) * ck_elems);
+		if (e == cudaErrorMemoryAllocation && s->ckseg < LG_SEG) {
+			cudaGetLastError();
+			s->ckseg *= 2;
+			checkpoint_offsets(s);
+			continue;
+		}
+		ok = shtb_cuda_ok(e, "checkpoints");
+		break;
+	}
 	// per-order ints
 	std::vector<int> mi(6 * (size_t) nm);
 	for (int im = 0; im < nm; im++) {
@@ -401,13 +431,10 @@ static int init_device(shtns_cfg s)
 		long double a = 2.0L * 3.14159265358979323846264338327950288L * (long double) j / (long double) s->nphi;
 		tw[j] = make_double2((double) std::cos(a), (double) std::sin(a));
 	}
-	const size_t ck_elems = (size_t) s->segtot * n2;
-	bool ok = true;
-	ok &= shtb_cuda_ok(cudaMalloc(&s->d_x, sizeof(double) * g.size()), "grid tables");
+	ok &= ok && shtb_cuda_ok(cudaMalloc(&s->d_x, sizeof(double) * g.size()), "grid tables");
 	ok &= ok && shtb_cuda_ok(cudaMalloc(&s->d_c, sizeof(double) * nc), "coefficient tables");
 	ok &= ok && shtb_cuda_ok(cudaMalloc(&s->d_mint, sizeof(int) * mi.size()), "order tables");
 	ok &= ok && shtb_cuda_ok(cudaMalloc(&s->d_tw, sizeof(double2) * tw.size()), "twiddles");
-	ok &= ok && shtb_cuda_ok(cudaMalloc(&s->d_ck, sizeof(double2) * ck_elems), "checkpoints");
 	int f1, f2;
 	if (ok && fft_fourstep_factors(s->nphi, f1, f2)) {
 		// factor tables of the four-step FFT
@@ -561,23 +588,16 @@ extern "C" int shtns_set_grid_auto(shtns_cfg s, enum shtns_type flags, double ep
 			s->tm_h[im] = it < s->nlat_2 ? it : s->nlat_2;
 		}
 	}
-	// recurrence checkpoints every 8 degree-pairs when they take at most
-	// 512 MB, every 16 up to 16 GB and an eighth of the GPU's memory (lmax 4095:
-	// 13.2 GB; 25.5 and 24.7 ms against 28.6 and 26.1 ms at 32 for the Legendre
-	// stages of 8 fields, whose tiles are generated in chains of one segment),
-	// else every 32
-	for (s->ckseg = 8; s->ckseg < LG_SEG; s->ckseg *= 2) {
+	// recurrence checkpoints: the table's bytes at spacings 8, 16 and 32
+	double bytes[3];
+	for (int i = 0; i < 3; i++) {
 		long segs = 0;
-		for (int im = 0; im <= s->mmax; im++) segs += (s->kmax_h[im] + s->ckseg - 1) / s->ckseg;
-		const double bytes = (double) segs * s->nlat_2 * 16.0;
-		double limit = 512.0 * 1024 * 1024;
-		if (s->ckseg > 8) {
-			size_t mem_free = 0, mem_total = 0;
-			if (cudaMemGetInfo(&mem_free, &mem_total) != cudaSuccess) { cudaGetLastError(); mem_total = 0; }
-			limit = std::min(16.0 * 1024 * 1024 * 1024, 0.125 * mem_total);
-		}
-		if (bytes <= limit) break;
+		for (int im = 0; im <= s->mmax; im++) segs += (s->kmax_h[im] + (8 << i) - 1) / (8 << i);
+		bytes[i] = (double) segs * s->nlat_2 * 16.0;
 	}
+	size_t mem_free = 0, mem_total = 0;
+	if (bytes[1] > CK_SMALL && cudaMemGetInfo(&mem_free, &mem_total) != cudaSuccess) { cudaGetLastError(); mem_free = 0; }
+	s->ckseg = shtns_b200_checkpoint_spacing(bytes, (double) mem_free);
 	checkpoint_offsets(s);
 	if (init_device(s) != 0) { plan_error("GPU initialisation failed: " + g_last_error); return -1; }
 	s->grid_set = 1;

@@ -59,3 +59,27 @@ def test_truncations_equal_zeroed_coefficients(comps, nf, ltr):
     for a, b in zip(tup(sh.analys(*v)), tup(sh.analys(*v, ltr=ltr))):
         assert float((a - b)[:, l <= ltr].abs().max()) <= 1e-13 * float(a.abs().max())
         assert not b[:, l > ltr].any()
+
+
+@pytest.mark.parametrize("lmax,free_mb,table_mb,seg", [(1023, 5000, 403, 8), (2047, 3000, 1610, 32), (1023, 380, 403, 16)])
+def test_plans_on_a_used_gpu(lmax, free_mb, table_mb, seg):
+    """The checkpoint table (table_mb: at the spacing that an empty GPU would
+    give) on a GPU with free_mb left: as dense as ever where it is small, coarser
+    where it would take more than a quarter, and at the next spacing where the
+    allocation fails.  The transforms are the same: bar as for any round trip."""
+    import shtns_b200
+    from shtns_b200 import capi
+    lib = capi.load()
+    dev = torch.device("cuda:0")
+    sh = shtns_b200.sht(lmax)
+    nlat = 3 * (lmax + 1) // 2
+    lib.shtns_b200_status()
+    torch.cuda.empty_cache()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - (free_mb << 20), dtype=torch.uint8, device=dev)
+    sh.set_grid(nlat, 2 * nlat, flags=shtns_b200.sht_quick_init | shtns_b200.SHT_THETA_CONTIGUOUS, polar_opt=1e-10)
+    del hold
+    torch.cuda.empty_cache()
+    assert lib.shtns_b200_get_option(sh._cfg, 2) == seg
+    assert lib.shtns_b200_status() == 0
+    q = torch.from_numpy(rand_spec(lmax, lmax, 1, 3)).to(dev)
+    assert relerr(q.cpu().numpy(), sh.analys(sh.synth(q)).cpu().numpy()) < 1e-11

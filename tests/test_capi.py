@@ -147,6 +147,22 @@ def test_plan_options_validate_and_read_back():
     lib.shtns_destroy(cfg)
 
 
+MB, GB = 2.0 ** 20, 2.0 ** 30
+
+
+@pytest.mark.parametrize("b8,free,want", [
+    (0.4 * GB, 100 * GB, 8), (0.4 * GB, 0.0, 8),             # small tables whatever is free
+    (0.9 * GB, 0.0, 16),                                     # 450 MB at 16
+    (3.2 * GB, 100 * GB, 16), (3.2 * GB, 6.5 * GB, 16),      # 1.6 GB: a quarter of what is free
+    (3.2 * GB, 6.3 * GB, 32), (3.2 * GB, 0.0, 32),
+    (26.4 * GB, 170 * GB, 16), (26.4 * GB, 50 * GB, 32),     # lmax 4095 on an empty and on a used GPU
+    (40.0 * GB, 1000 * GB, 32)])                             # beyond 16 GB
+def test_checkpoint_spacing_by_table_size_and_free_memory(b8, free, want):
+    lib = capi.load()
+    bytes3 = (C.c_double * 3)(b8, b8 / 2, b8 / 4)
+    assert lib.shtns_b200_checkpoint_spacing(bytes3, free) == want
+
+
 def test_public_headers_compile_as_c99_and_cxx():
     """include/shtns.h, shtns_cuda.h and shtns_b200.h compile in a C99 unit
     (complex.h cplx, enums, extern "C" guards) and in a C++ unit, and the C
