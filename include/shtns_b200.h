@@ -160,8 +160,9 @@ size_t shtns_b200_split_table_bytes(shtns_cfg);
  * plan i (device pointers; spec_dist = nlm, spat_dist = nspat of that plan).
  * All launches are ordered by the compute stream of the first plan, so a call
  * can be captured in a CUDA graph (after one call with the same field counts,
- * which allocates the work buffers and the work list).  Plans in a group get a
- * common checkpoint spacing.  No counterpart in SHTns 3.5.2. */
+ * which allocates the work buffers and the work list).  Plans keep their
+ * checkpoint spacing; the persistent launch reads every table at the largest
+ * spacing among them.  No counterpart in SHTns 3.5.2. */
 typedef struct shtns_b200_group* shtns_group;
 shtns_group shtns_b200_group_create(int nplans, shtns_cfg* plans);
 void shtns_b200_group_destroy(shtns_group);
@@ -176,6 +177,8 @@ void shtns_b200_group_destroy(shtns_group);
  * stream (with option 4 = 1 the plans run concurrently), 0 one persistent
  * launch over all plans (options 1 and 2 are its own).  Return 0 or -1. */
 int shtns_b200_group_set_option(shtns_group, int option, int value);
+/* Current value of option 1, 2, 4 or 5; -1 otherwise. */
+int shtns_b200_group_get_option(shtns_group, int option);
 void shtns_b200_group_synth(shtns_group, cplx **Qlm, double **Vr, const int *nfields, int ltr);
 void shtns_b200_group_analys(shtns_group, double **Vr, cplx **Qlm, const int *nfields, int ltr);
 /* Vector transforms of a group (the plans' SHsphtor / SHqst forms): per plan

@@ -64,6 +64,9 @@ class PlanGroup:
         if self._lib.shtns_b200_group_set_option(self._g, int(option), int(value)) != 0:
             raise ValueError("invalid group option %d = %d" % (option, value))
 
+    def get_option(self, option):
+        return self._lib.shtns_b200_group_get_option(self._g, int(option))
+
     def _args(self, src, dst):
         n = len(self.plans)
         A = (C.c_void_p * n)(*[x.data_ptr() if x is not None else 0 for x in src])

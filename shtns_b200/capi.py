@@ -141,6 +141,7 @@ PROTOTYPES = {
     "shtns_b200_group_create": (P, [I, P]),
     "shtns_b200_group_destroy": (None, [P]),
     "shtns_b200_group_set_option": (I, [P, I, I]),
+    "shtns_b200_group_get_option": (I, [P, I]),
     "shtns_b200_group_synth": (None, [P, P, P, P, I]),
     "shtns_b200_group_analys": (None, [P, P, P, P, I]),
     "shtns_b200_group_SHsphtor_to_spat": (None, [P, P, P, P, P, P, I]),

@@ -622,7 +622,6 @@ struct GroupWork {
 
 struct shtns_b200_group {
 	std::vector<shtns_cfg> plans;
-	int ckseg;
 	int order;                       // 0: work items by decreasing cost, 1: plan/order/tile order
 	int nsm;
 	int ctas_per_sm;                 // CTAs of the persistent launch per SM (1-3)
@@ -680,6 +679,17 @@ bool group_may_rewrite(cudaStream_t st)
 		return false;
 	}
 	return shtb_cuda_ok(cudaStreamSynchronize(st), "plan group stream");
+}
+
+// One instance of the persistent kernel serves all plans: segments of the
+// largest spacing among the plans, which read every second or fourth
+// checkpoint of a denser table.  Returns that spacing.
+int group_spacing(std::vector<LegParams>& lp)
+{
+	int seg = 8;
+	for (const LegParams& p : lp) seg = std::max(seg, p.ckseg);
+	for (LegParams& p : lp) p = leg_spaced(p, seg);
+	return seg;
 }
 
 // build (or reuse) the work list of the persistent Legendre launch
@@ -767,21 +777,12 @@ bool group_work(shtns_group g, const std::vector<LegParams>& lp, const int* nfie
 extern "C" shtns_group shtns_b200_group_create(int nplans, shtns_cfg* plans)
 {
 	if (nplans < 1 || !plans) { shtb_set_error(1, "shtns_b200_group_create: no plans"); return nullptr; }
-	int seg = plans[0] ? plans[0]->ckseg : 0;
 	for (int i = 0; i < nplans; i++) {
 		if (!plans[i] || !plans[i]->grid_set) { shtb_set_error(1, "shtns_b200_group_create: plan without grid"); return nullptr; }
 		if (plans[i]->dev != plans[0]->dev) { shtb_set_error(1, "shtns_b200_group_create: plans on different devices"); return nullptr; }
-		seg = std::max(seg, plans[i]->ckseg);
 	}
-	// one persistent kernel instance serves all plans: same checkpoint spacing
-	for (int i = 0; i < nplans; i++)
-		if (plans[i]->ckseg != seg && shtns_b200_set_option(plans[i], 2, seg) != 0) {
-			shtb_set_error(1, "shtns_b200_group_create: cannot align checkpoint spacing");
-			return nullptr;
-		}
 	shtns_group g = new shtns_b200_group();
 	g->plans.assign(plans, plans + nplans);
-	g->ckseg = seg;
 	g->order = 0;
 	g->ctas_per_sm = 3;
 	g->concurrent = 1;
@@ -828,10 +829,21 @@ extern "C" int shtns_b200_group_set_option(shtns_group g, int option, int value)
 	if (option == 3 && (value == 8 || value == 16 || value == 32)) {
 		for (shtns_cfg s : g->plans)
 			if (s->ckseg != value && shtns_b200_set_option(s, 2, value) != 0) return -1;
-		g->ckseg = value;
 		return 0;
 	}
 	return -1;
+}
+
+extern "C" int shtns_b200_group_get_option(shtns_group g, int option)
+{
+	if (!g) return -1;
+	switch (option) {
+		case 1: return g->order;
+		case 2: return g->ctas_per_sm;
+		case 4: return g->concurrent;
+		case 5: return g->leg_per_plan;
+		default: return -1;
+	}
 }
 
 namespace {
@@ -879,10 +891,11 @@ void group_synth_impl(shtns_group g, int ncomp, const int* types, cplx** const* 
 		check_launch("group synthesis launch");
 		return;
 	}
+	const int seg = group_spacing(lp);
 	if (!group_work(g, lp, nfields, true)) return;
 	group_fork(g, st, nfields, prologue);
 	const GroupWork& W = g->dir[1];
-	launch_leg_multi(W.d_plist, W.d_work, W.nwork, W.d_counter, g->ckseg, true, g->nsm * g->ctas_per_sm, st);
+	launch_leg_multi(W.d_plist, W.d_work, W.nwork, W.d_counter, seg, true, g->nsm * g->ctas_per_sm, st);
 	group_fork(g, st, nfields, fft);
 	check_launch("group synthesis launch");
 }
@@ -929,10 +942,11 @@ void group_analys_impl(shtns_group g, int ncomp, const int* types, double** cons
 		check_launch("group analysis launch");
 		return;
 	}
+	const int seg = group_spacing(lp);
 	if (!group_work(g, lp, nfields, false)) return;
 	group_fork(g, st, nfields, fft);
 	const GroupWork& W = g->dir[0];
-	launch_leg_multi(W.d_plist, W.d_work, W.nwork, W.d_counter, g->ckseg, false, g->nsm * g->ctas_per_sm, st);
+	launch_leg_multi(W.d_plist, W.d_work, W.nwork, W.d_counter, seg, false, g->nsm * g->ctas_per_sm, st);
 	group_fork(g, st, nfields, epilogue);
 	check_launch("group analysis launch");
 }

@@ -173,6 +173,44 @@ def test_autotune_options_agree(small, tmp_path):
     assert rec2["options"] == rec["options"] and ub.options == rec["options"]
 
 
+def test_group_leaves_the_plans_checkpoint_spacing():
+    """A group of plans with different spacings, one of them with a clone that is
+    in the group too: the tables stay as they are, and the persistent launch,
+    which reads each of them at the largest spacing, gives the per-plan results."""
+    import shtns_b200
+    from shtns_b200 import batch as B
+    from shtns_b200 import capi
+    lib = capi.load()
+    plans = []
+    for lmax, seg in ((63, 8), (95, 32), (127, 16)):
+        sh = shtns_b200.sht(lmax)
+        sh.set_grid(*B.grid_for(lmax), flags=shtns_b200.sht_quick_init | shtns_b200.SHT_THETA_CONTIGUOUS, polar_opt=1e-10)
+        assert lib.shtns_b200_set_option(sh._cfg, 2, seg) == 0
+        plans.append(sh)
+    plans.append(plans[0].clone())
+    segs = [8, 32, 16, 8]
+    g = B.PlanGroup(plans)
+    assert [lib.shtns_b200_get_option(sh._cfg, 2) for sh in plans] == segs
+    dev = torch.device("cuda:0")
+    q = [torch.from_numpy(rand_spec(sh.lmax, sh.lmax, 1, 60 + i, nfields=3 + i)).to(dev) for i, sh in enumerate(plans)]
+    out = {}
+    for form in (1, 0):
+        g.set_option(5, form)
+        assert g.get_option(5) == form
+        v = [torch.full((x.shape[0],) + sh.spat_shape, float("nan"), dtype=torch.float64, device=dev) for x, sh in zip(q, plans)]
+        r = [torch.full_like(x, float("nan")) for x in q]
+        g.synth_into(q, v)
+        g.analys_into(v, r)
+        torch.cuda.synchronize()
+        out[form] = v + r
+        assert [lib.shtns_b200_get_option(sh._cfg, 2) for sh in plans] == segs
+        for a, b in zip(q, r):
+            assert relerr(a.cpu().numpy(), b.cpu().numpy()) < 1e-12
+    for a, b in zip(out[0], out[1]):
+        assert float((a - b).abs().max() / a.abs().max()) < 1e-13
+    g.close()
+
+
 def test_uneven_full_workload_roundtrip():
     """256 fields, lmax uniform in {63,...,1023}: group and graph round trips."""
     lm = np.random.default_rng(2024).choice((63, 127, 255, 511, 1023), size=256)
