@@ -263,13 +263,20 @@ class UnevenBatch:
 
     # ---------------- options ----------------
     def apply_options(self, opts):
-        """opts: {"fft_pairs": [per bucket], "ckseg": c, "order": o, "ctas_per_sm": k}."""
+        """opts: {"fft_pairs": [per bucket], "ckseg": c or [per bucket], "order": o,
+        "ctas_per_sm": k} (the last two count in the persistent form only)."""
         lib = capi.load()
         for sh, S in zip(self.plans, opts.get("fft_pairs", [])):
             if lib.shtns_b200_set_option(sh._cfg, 1, int(S)) != 0:
                 raise ValueError("invalid FFT pairs %r" % S)
         if "ckseg" in opts:
-            self.group.set_option(3, opts["ckseg"])
+            seg = opts["ckseg"]
+            if isinstance(seg, (list, tuple)):
+                for sh, c in zip(self.plans, seg):
+                    if lib.shtns_b200_set_option(sh._cfg, 2, int(c)) != 0:
+                        raise ValueError("invalid checkpoint spacing %r" % c)
+            else:
+                self.group.set_option(3, seg)
         if "order" in opts:
             self.group.set_option(1, opts["order"])
         if "ctas_per_sm" in opts:
@@ -302,12 +309,16 @@ def autotune(batch, reps=3, cache=None, use_cache=True, log=None):
     """Choose the options of an UnevenBatch by timing them on the device.
 
     Search: for each bucket, latitude pairs per FFT CTA in {1, 2, 4, 8}, timed on
-    that bucket's batched transforms; then for the group, checkpoint spacing
-    in {8, 16, 32} x work order {cost, natural} x CTAs per SM {2, 3}, timed on
-    pair().  The choice is applied, cached (JSON, keyed by device name and the
+    that bucket's batched transforms; then for the group, timed on pair(): in
+    the per-plan form (group option 5 = 1, the default) the plans' own checkpoint
+    spacings and a common one in {8, 16, 32}; in the persistent form common
+    spacing in {8, 16, 32} x work order {cost, natural} x CTAs per SM {2, 3}.
+    The choice is applied, cached (JSON, keyed by device name, form and the
     (lmax, fields) of each bucket) and returned with the timings."""
+    lib = capi.load()
+    persistent = batch.group.get_option(5) == 0
     dev = torch.cuda.get_device_name(batch.device)
-    key = dev + "|" + ",".join("%dx%d" % (l, n) for l, n in zip(batch.buckets, batch.count))
+    key = dev + ("|persistent|" if persistent else "|per plan|") + ",".join("%dx%d" % (l, n) for l, n in zip(batch.buckets, batch.count))
     path = _cache_path(cache)
     db = {}
     if use_cache and os.path.exists(path):
@@ -320,7 +331,6 @@ def autotune(batch, reps=3, cache=None, use_cache=True, log=None):
         batch.apply_options(db[key]["options"])
         return db[key]
     trials = []
-    lib = capi.load()
     pairs = []
     for b, sh in enumerate(batch.plans):
         q, v, r = batch.Q[b], batch.V[b], batch.R[b]
@@ -338,17 +348,19 @@ def autotune(batch, reps=3, cache=None, use_cache=True, log=None):
         pairs.append(best[1])
         lib.shtns_b200_set_option(sh._cfg, 1, best[1])
     best = None
-    for seg in (8, 16, 32):
-        for order in (0, 1):
-            for k in (2, 3):
-                opts = {"fft_pairs": pairs, "ckseg": seg, "order": order, "ctas_per_sm": k}
-                batch.apply_options(opts)
-                t = _time(batch.pair, reps)
-                trials.append(dict(opts, ms=t))
-                if log:
-                    log("autotune %s: %.3f ms" % (opts, t))
-                if best is None or t < best[0]:
-                    best = (t, opts)
+    if persistent:
+        tries = [{"ckseg": seg, "order": order, "ctas_per_sm": k} for seg in (8, 16, 32) for order in (0, 1) for k in (2, 3)]
+    else:
+        tries = [{"ckseg": seg} for seg in ([lib.shtns_b200_get_option(sh._cfg, 2) for sh in batch.plans], 8, 16, 32)]
+    for o in tries:
+        opts = dict(o, fft_pairs=pairs)
+        batch.apply_options(opts)
+        t = _time(batch.pair, reps)
+        trials.append(dict(opts, ms=t))
+        if log:
+            log("autotune %s: %.3f ms" % (opts, t))
+        if best is None or t < best[0]:
+            best = (t, opts)
     batch.apply_options(best[1])
     rec = {"options": best[1], "ms": best[0], "trials": trials}
     db[key] = rec

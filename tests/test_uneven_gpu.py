@@ -1,5 +1,6 @@
-"""Fields of uneven lmax through a plan group (one persistent Legendre launch
-per direction), its CUDA-graph replay and the autotuner.
+"""Fields of uneven lmax through a plan group (each plan's own kernels, or one
+persistent Legendre launch per direction), its CUDA-graph replay and the
+autotuner.
 
 Checks, on seeded N(0,1)/(l+1) coefficients:
   * group synthesis and analysis equal the per-bucket batched cu_* transforms
@@ -142,7 +143,7 @@ def test_group_per_plan_legendre_form(small, concurrent):
             assert float((a - b).abs().max() / a.abs().max()) < 1e-14
         ub.release_graph()
     finally:
-        ub.group.set_option(5, 0)
+        ub.group.set_option(5, 1)
         ub.group.set_option(4, 1)
 
 
@@ -154,6 +155,7 @@ def test_autotune_options_agree(small, tmp_path):
     torch.cuda.synchronize()
     V0, R0 = [v.clone() for v in ub.V], [r.clone() for r in ub.R]
     path = str(tmp_path / "tune.json")
+    ub.group.set_option(5, 0)                # the persistent form, which has work order and CTAs per SM
     rec = B.autotune(ub, reps=1, cache=path)
     assert set(rec["options"]) == {"fft_pairs", "ckseg", "order", "ctas_per_sm"}
     assert len(rec["trials"]) == 4 * len(ub.plans) + 12
@@ -171,6 +173,10 @@ def test_autotune_options_agree(small, tmp_path):
     # cached choice is applied without timing
     rec2 = B.autotune(ub, cache=path)
     assert rec2["options"] == rec["options"] and ub.options == rec["options"]
+    # the per-plan form is searched for itself
+    ub.group.set_option(5, 1)
+    rec3 = B.autotune(ub, reps=1, cache=path)
+    assert set(rec3["options"]) == {"fft_pairs", "ckseg"} and len(rec3["trials"]) == 4 * len(ub.plans) + 4
 
 
 def test_group_leaves_the_plans_checkpoint_spacing():
