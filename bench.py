@@ -671,12 +671,38 @@ def uneven_flops(batch):
     return 2 * tot
 
 
+def uneven_group_forms(ub, timed, steps, autotune):
+    """Times the plan group's two forms, each with its own options: the per-plan
+    kernels (group option 5 = 1), then one persistent Legendre launch (0).  Leaves
+    the batch in the faster form, captured; returns (its name, {form: {"eager",
+    "eager_one_stream", "graph": ms, "options"}})."""
+    out = {}
+    for name, opt in (("per_plan", 1), ("persistent", 0)):
+        ub.release_graph()
+        ub.group.set_option(5, opt)
+        rec = {"options": autotune(ub)}
+        ub.group.set_option(4, 0)          # every launch of the group on one stream
+        rec["eager_one_stream"] = timed(ub.pair, steps)
+        ub.group.set_option(4, 1)          # per-plan launches concurrently on side streams (default)
+        rec["eager"] = timed(ub.pair, steps)
+        ub.capture()
+        rec["graph"] = timed(ub.replay, steps)
+        out[name] = rec
+    best = min(out, key=lambda k: out[k]["graph"])
+    ub.release_graph()
+    ub.group.set_option(5, 1 if best == "per_plan" else 0)
+    ub.apply_options(out[best]["options"])
+    ub.capture()
+    return best, out
+
+
 def run_uneven(args):
     """256 scalar fields, lmax uniform in {63,...,1023}, each on its own Gauss
     grid nlat=3(lmax+1)/2, nphi=2 nlat: one step = synthesis + analysis of all
     fields.  Forms timed: one cu_* pair per field, one batched pair per lmax
-    bucket, the plan group (one persistent Legendre launch per direction)
-    eagerly, and the plan group replayed from a CUDA graph (the value)."""
+    bucket, the plan group eagerly and replayed from a CUDA graph, with each
+    plan's own Legendre kernels and with one persistent Legendre launch per
+    direction; the value is the faster graph."""
     import torch
     torch.cuda.set_device(0)
     dev = torch.device("cuda", 0)
@@ -687,7 +713,6 @@ def run_uneven(args):
     ub = B.UnevenBatch(lm, device=dev, polar_opt=EPS)
     for b, (l, n) in enumerate(zip(ub.buckets, ub.count)):
         ub.Q[b].copy_(torch.from_numpy(rand_spec(l, l, 1, 300 + b, power=1.0, nfields=n)))
-    tune = B.autotune(ub, use_cache=False)
 
     def timed(fn, steps):
         for _ in range(args.warmup):
@@ -703,34 +728,15 @@ def run_uneven(args):
 
     from shtns_b200 import capi
     lib = capi.load()
-    ms_field = timed(ub.pair_per_field, max(3, args.steps // 20))
-    ms_bucket = timed(ub.pair_per_bucket, args.steps)
-    ub.group.set_option(4, 0)          # every launch of the group on one stream
-    ms_group1 = timed(ub.pair, args.steps)
-    ub.group.set_option(4, 1)          # per-plan launches concurrently on side streams (default)
-    ms_group = timed(ub.pair, args.steps)
-    ub.capture()
-    torch.cuda.synchronize()
     clocks = ClockSampler(0)
     clocks.start()
     time.sleep(0.3)
-    ms_graph_persistent = timed(ub.replay, args.steps)
-    ub.release_graph()
-    # each bucket's own kernels, the buckets concurrently on the group's side
-    # streams, captured as parallel branches of one graph
-    ub.group.set_option(5, 1)
-    ms_group_pp = timed(ub.pair, args.steps)
-    ub.capture()
+    form, forms = uneven_group_forms(ub, timed, args.steps, lambda b: B.autotune(b, use_cache=False)["options"])
     torch.cuda.synchronize()
-    ms_graph_pp = timed(ub.replay, args.steps)
     clk = clocks.stop()
-    per_plan = ms_graph_pp < ms_graph_persistent
-    ms_graph = min(ms_graph_pp, ms_graph_persistent)
-    if not per_plan:
-        ub.release_graph()
-        ub.group.set_option(5, 0)
-        ub.capture()
-        torch.cuda.synchronize()
+    ms_graph = forms[form]["graph"]
+    ms_field = timed(ub.pair_per_field, max(3, args.steps // 20))
+    ms_bucket = timed(ub.pair_per_bucket, args.steps)
     n0 = lib.shtns_b200_launch_count()
     ub.pair()
     torch.cuda.synchronize()
@@ -748,19 +754,20 @@ def run_uneven(args):
                    "grids": {str(l): list(B.grid_for(l)) for l in ub.buckets}, "polar_eps": EPS,
                    "layout": "theta-contiguous",
                    "form": "plan group replayed from a CUDA graph (%s)" % (
-                       "per-bucket kernels on concurrent graph branches" if per_plan else
+                       "per-bucket kernels on concurrent graph branches" if form == "per_plan" else
                        "one persistent Legendre launch")},
         "forms_fields_per_s": {"per_field_launches": nf / (ms_field * 1e-3),
                                "per_bucket_batched": nf / (ms_bucket * 1e-3),
-                               "group_eager_one_stream": nf / (ms_group1 * 1e-3),
-                               "group_eager": nf / (ms_group * 1e-3),
-                               "group_cuda_graph_persistent_legendre": nf / (ms_graph_persistent * 1e-3),
-                               "group_eager_per_bucket_kernels_concurrent": nf / (ms_group_pp * 1e-3),
-                               "group_cuda_graph_per_bucket_kernels_concurrent": nf / (ms_graph_pp * 1e-3),
+                               "group_eager_one_stream": nf / (forms["persistent"]["eager_one_stream"] * 1e-3),
+                               "group_eager": nf / (forms["persistent"]["eager"] * 1e-3),
+                               "group_cuda_graph_persistent_legendre": nf / (forms["persistent"]["graph"] * 1e-3),
+                               "group_eager_per_bucket_kernels_one_stream": nf / (forms["per_plan"]["eager_one_stream"] * 1e-3),
+                               "group_eager_per_bucket_kernels_concurrent": nf / (forms["per_plan"]["eager"] * 1e-3),
+                               "group_cuda_graph_per_bucket_kernels_concurrent": nf / (forms["per_plan"]["graph"] * 1e-3),
                                "group_cuda_graph": nf / (ms_graph * 1e-3)},
         "speedup_vs_per_field": ms_field / ms_graph,
-        "autotune": tune["options"],
-        "roofline": {"kernel": "whole step (Legendre flops / step time: lower bound for leg_multi_kernel)",
+        "autotune": {k: f["options"] for k, f in forms.items()},
+        "roofline": {"kernel": "whole step (Legendre flops / step time: lower bound for the Legendre kernels)",
                      "bound": "tensor", "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak,
                      "traffic": None, "peak_source": "measured in this run: cuBLAS DGEMM 8192^3"},
         "roundtrip_relerr": rt,

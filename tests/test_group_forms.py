@@ -1,5 +1,6 @@
-"""CPU check of the autotuner on a stand-in for the device batch: it searches
-only options that count in the plan group's current form."""
+"""CPU checks of what chooses between the plan group's two forms: the autotuner
+searches only options that count in the current form, and bench.py times each
+form with the option that selects it, on a stand-in for the device batch."""
 import types
 
 import pytest
@@ -47,3 +48,20 @@ def test_autotune_searches_the_options_of_the_current_form(form, tmp_path, monke
     other = FakeBatch(1 - form)
     assert set(B.autotune(other, cache=path)["options"]) != set(rec["options"])
     assert B.autotune(FakeBatch(form), cache=path)["options"] == rec["options"]
+
+
+@pytest.mark.parametrize("fast", [0, 1])
+def test_bench_times_each_form_with_its_own_option(fast):
+    import bench
+    ub = FakeBatch(1)
+
+    def timed(fn, steps):
+        fn()
+        what, form, _ = ub.log[-1]
+        return 1.0 if form == fast else 2.0
+    best, forms = bench.uneven_group_forms(ub, timed, 1, lambda b: {"form": b.options[5]})
+    assert ub.log == [("pair", 1, 0), ("pair", 1, 1), ("graph", 1, 1), ("pair", 0, 0), ("pair", 0, 1), ("graph", 0, 1)]
+    assert best == ("per_plan" if fast else "persistent")
+    # the batch is left in the form that is reported, with that form's options
+    assert ub.options[5] == fast and ub.captured == fast and ub.applied == {"form": fast}
+    assert forms["per_plan"]["options"] == {"form": 1} and forms["persistent"]["options"] == {"form": 0}
