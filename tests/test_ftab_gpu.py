@@ -5,9 +5,10 @@ results agree bit for bit.  Cases: vector (qst) fields with a polar
 threshold, a truncated call (ltr < lmax: coefficient rows beyond the call's
 last step are zeros), a column tile that is not full, a grid whose half
 latitude count is not a multiple of 32, and the automatic mode (option 10 =
-0), which takes the table for these sizes; an mres = 2 plan, the adjoint of
-the analysis (the same launch with row weights) and clones made before and
-after the table is built (they use the base plan's table)."""
+0) below and above the 33 field-components from which it takes the table; an
+mres = 2 plan, the adjoint of the analysis (the same launch with row weights)
+and clones made before and after the table is built (they use the base plan's
+table)."""
 import numpy as np
 import pytest
 
@@ -37,10 +38,10 @@ def _both(sh, fn):
 
 
 @pytest.mark.parametrize("L,nlat,nphi,eps", [(255, 384, 768, 1e-10), (200, 304, 600, 0.0)])
-def test_table_synthesis_bit_identical_qst(L, nlat, nphi, eps):
+@pytest.mark.parametrize("nf", [7, 11])                 # 21 and 33 field-components: the last column tile is partial
+def test_table_synthesis_bit_identical_qst(L, nlat, nphi, eps, nf):
     dev = torch.device("cuda:0")
     sh = _plan(L, nlat, nphi, eps)
-    nf = 7                                              # 21 field-components: the last column tile is partial
     q = torch.from_numpy(rand_spec(L, L, 1, 31, power=1.0, nfields=nf)).to(dev)
     s = torch.from_numpy(rand_spec(L, L, 1, 32, power=1.5, zero_l0=True, nfields=nf)).to(dev)
     t = torch.from_numpy(rand_spec(L, L, 1, 33, power=1.5, zero_l0=True, nfields=nf)).to(dev)
@@ -48,6 +49,22 @@ def test_table_synthesis_bit_identical_qst(L, nlat, nphi, eps):
     for mode in (2, 0):
         for a, b in zip(out[mode], out[1]):
             assert torch.equal(a, b)
+
+
+def test_automatic_mode_builds_the_table_from_33_components():
+    from shtns_b200 import capi
+    lib = capi.load()
+    sh = _plan(127, 192, 384, 1e-10)
+    q = torch.from_numpy(rand_spec(127, 127, 1, 36, power=1.0, nfields=33)).to(torch.device("cuda:0"))
+    assert lib.shtns_b200_set_option(sh._cfg, 10, 1) == 0
+    sh.synth(q)                               # work buffers
+    assert lib.shtns_b200_set_option(sh._cfg, 10, 0) == 0
+    b = lib.shtns_b200_device_bytes(sh._cfg)
+    sh.synth(q[:32])
+    assert lib.shtns_b200_device_bytes(sh._cfg) == b
+    sh.synth(q)
+    assert lib.shtns_b200_device_bytes(sh._cfg) > b + 1_000_000
+    assert sh.kernel_errors() == 0
 
 
 def test_table_synthesis_truncated_and_scalar():
