@@ -13,8 +13,9 @@
 //
 // The product runs on the FP64 tensor cores (mma.sync m16n8k4 f64: tcgen05 has
 // no FP64 kind).  Each CTA regenerates its Y tile in shared memory from
-// recurrence checkpoints (Y_k, Y_{k+1}) stored every 32 degrees, so tiles can
-// start at any k and the recurrence of one tile is only 32 dependent steps.
+// recurrence checkpoints (Y_k, Y_{k+1}) stored every 8, 16 or 32 steps k, so
+// tiles can start at any k and a thread's part of the recurrence is as short
+// as one segment (leg_spaced picks the segments of a launch).
 #include "sht_internal.h"
 #include "sht_legendre_tiles.h"
 

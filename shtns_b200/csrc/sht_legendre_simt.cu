@@ -1,11 +1,14 @@
-// SIMT FP64 Legendre kernels for calls with few field-components (1 to 4).
+// SIMT FP64 Legendre kernels for calls with few field-components: by default the
+// synthesis of one to three (three on grids of more than 1024 rows) and the
+// analysis of one, with option 5 = 8 up to four (leg_simt_selected).
 //
 // The tensor-core tiles (sht_legendre.cu) multiply the on-the-fly Y tile by 16
 // GEMM columns per group of 4 field-components; with one field 12 of the 16
 // columns are padding.  On sm_100a the FP64 FMA pipe has the throughput of the
-// FP64 tensor path, so for one to four field-components these kernels do the
-// minimum work instead: per (row, k) two FMAs of recurrence and four FMAs per
-// field-component, with Y never leaving registers in the synthesis.
+// FP64 tensor path, so these kernels do the minimum work instead: per (row, k)
+// two FMAs of recurrence and four FMAs per field-component, with Y never
+// leaving registers in the synthesis.  With more components the reads of
+// coefficients or of Y from shared memory cost more than the padding.
 //
 // Same recurrence, checkpoints and coefficient layout as the tensor-core
 // kernels (the reference's SHT/kernel_SH_to_spat.gen.c:388-441 and
@@ -307,11 +310,9 @@ __global__ void __launch_bounds__(SA_NT) leg_analys_simt_kernel(LegParams p)
 // when the block starts inside a segment) and accumulates Y_k G for its rows:
 // 4 x 16 = 64 sums per thread.  They are reduced once per CTA: a butterfly
 // reduce-scatter inside each warp (lane L ends with sums 2L and 2L+1), then
-// across the two warps in shared memory.  Measured on B200 against the
-// shared-memory kernel above: faster for one component when the checkpoints
-// are 16 or 32 apart or the grid has at most 1024 rows (2x at lmax 127, 1.5x at
-// 511, 1.15x at 4095), slower at lmax 1023 (checkpoints 8 apart) and for two
-// components.
+// across the two warps in shared memory.  Segments of 32 steps, whatever the
+// table's spacing.  With two or more components the sums no longer fit the
+// registers (tensor-core tiles, or the shared-memory kernel above).
 #define SR_NT 64
 #define SR_NV 64                       // partial sums per thread
 
