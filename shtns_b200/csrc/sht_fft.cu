@@ -732,7 +732,7 @@ bool launch_fft4(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 	} else {
 		// theta-contiguous grids only (phi-contiguous rows are read faster
 		// straight from global memory by the direct kernel)
-		if (!grid_ok) return false;
+		if (!grid_ok || (S == 1 && p.f32)) return false;      // a pair of floats is half of a tensor copy's 16 bytes
 		tt.box = box_j(N);
 		tt.ncopy = N / tt.box;
 		stage_bytes = (size_t) N * 2 * S * (p.f32 ? 4 : 8);
@@ -766,7 +766,8 @@ bool launch_fft4(const FftParams& p, int nfc, cudaStream_t st, bool synth)
 	};
 	if (synth) return p.f32 ? go(fft4_synth_kernel<N, S, false, float>)
 	                        : (tout ? go(fft4_synth_kernel<N, S, true, double>) : go(fft4_synth_kernel<N, S, false, double>));
-	return p.f32 ? go(fft4_analys_kernel<N, S, float>) : go(fft4_analys_kernel<N, S, double>);
+	if constexpr (S > 1) if (p.f32) return go(fft4_analys_kernel<N, S, float>);
+	return go(fft4_analys_kernel<N, S, double>);
 }
 
 template <int N, int S>
@@ -909,7 +910,7 @@ void set_fft4_limits(int lim)
 	set(fft4_synth_kernel<N, S, false, double>);
 	set(fft4_synth_kernel<N, S, false, float>);
 	set(fft4_analys_kernel<N, S, double>);
-	set(fft4_analys_kernel<N, S, float>);
+	if constexpr (S > 1) set(fft4_analys_kernel<N, S, float>);
 }
 
 template <int N, int S>
