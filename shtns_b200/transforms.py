@@ -290,15 +290,19 @@ class sht:
     def synth_into(self, q, outs, ltr=None):
         """Device synthesis into preallocated tensors (no allocation by torch):
         q: list of 1-3 complex128 CUDA tensors (..., nlm); outs: float64 (..., *spat_shape)."""
-        self._transform(len(q) - 1, q[0].numel() // self.nlm, q, outs, ltr)
+        n = min(len(q), 3)
+        self._transform(n - 1, q[0].numel() // self.nlm, q[:n], outs[:n], ltr)
 
     def analys_into(self, v, outs, ltr=None):
         """Device analysis into preallocated tensors (see synth_into)."""
-        self._transform(len(v) + 2, v[0].numel() // self.nspat, v, outs, ltr)
+        n = min(len(v), 3)
+        self._transform(n + 2, v[0].numel() // self.nspat, v[:n], outs[:n], ltr)
 
     def _transform(self, kind, nf, src, dst, ltr):
         """One device transform of nf fields on torch's current stream (kinds
         of shtns_b200_transform): one foreign call, as its cost counts on small fields."""
+        if len(dst) < len(src):         # the arrays that are not given are null
+            raise IndexError("%d components but %d output tensors" % (len(src), len(dst)))
         p = [x.data_ptr() for x in src] + [x.data_ptr() for x in dst]
         p += [None] * (6 - len(p))
         lib = self._lib
